@@ -1,5 +1,5 @@
 // K1-K3: octave base (luma->f32, 2x bilinear upsample, initial blur), separable
-// Gaussian blur chain + DoG, and the 2x decimation that seeds the next octave.
+// Gaussian blur chain, and the 2x decimation that seeds the next octave.
 //
 // Reference: gaussian_blur (src/pipeline.rs:314-425), upsample_2x_bilinear
 // (:455-483), downsample_2x (:429-449), build_scale_space_pyramid_with_options
@@ -27,9 +27,8 @@
 //   Taps are consumed in input order; for every output that is k = 0..2R, the
 //   reference's order.  The row-pair stride is 2 (mod 16) float2 and lanes are
 //   assigned so that the 8 lanes of a quarter-warp hit 8 distinct 16-byte bank
-//   groups.  Outputs: G_s and D_{s-1} = G_s - G_{s-1} as 64-bit stores; level
-//   `scales` also writes the even/even samples that form the next octave's base
-//   (fused downsample_2x).  Images alternate direction between consecutive
+//   groups.  Outputs: G_s as 64-bit stores; level `scales` also writes the
+//   even/even samples that form the next octave's base (fused downsample_2x).  Images alternate direction between consecutive
 //   levels (blockIdx.z reversed on odd levels) so the planes written last by
 //   one launch, still in L2, are read first by the next.
 #pragma once
@@ -203,8 +202,8 @@ __device__ __forceinline__ void prefetch_ahead_rows(const ImagePlan* __restrict_
 // One blur level for every image of the batch (blockIdx.z = image, reversed when
 // zrev; or, over images of different sizes, one CTA per existing tile of the
 // launch's tile work list, the list reversed when zrev).
-//   MODE_LEVEL: G[s] = blur(G[s-1]); D[s-1] = G[s] - G[s-1]; level `down_level` also
-//               writes the next octave's G[0] (even rows/columns).
+//   MODE_LEVEL: G[s] = blur(G[s-1]); level `down_level` also writes the next
+//               octave's G[0] (even rows/columns).
 //   MODE_INIT_*: G[0] of octave 0 from the input image.
 // TH x 64 tiles (TH = 64, or 128 for the tall variant), NT threads.
 template <int R, int HC, int RV, int MODE, bool FUSED, bool TILED, int TH = kTileH, int NT = kBlurThreads>
@@ -399,7 +398,6 @@ __device__ __forceinline__ void blur_level_body(const ImagePlan* __restrict__ pl
   // 3. Vertical pass: a column pair x RV rows per thread.
   const long long gbase = (long long)level * O.plane_stride;
   float* gout = O.g + gbase;
-  float* dout = (MODE == MODE_LEVEL) ? O.d + (long long)(level - 1) * O.plane_stride : nullptr;
   const bool do_down = (MODE == MODE_LEVEL) && level == down_level && octave + 1 < P.n_oct;
   const int x = 2 * lane;
   const int gx = tx0 + x;
@@ -419,13 +417,6 @@ __device__ __forceinline__ void blur_level_body(const ImagePlan* __restrict__ pl
     }
     if (gx >= w) continue;
     const bool pair_ok = gx + 1 < w;
-    constexpr int NPR = ((R & 1) + RV + 1) / 2;
-    float4 prevp[MODE == MODE_LEVEL ? NPR : 1];
-    if constexpr (MODE == MODE_LEVEL) {
-      const float4* pp = reinterpret_cast<const float4*>(s_in + ((R >> 1) + (yb >> 1)) * Gm::IN_S + Gm::RP + x);
-#pragma unroll
-      for (int p = 0; p < NPR; ++p) prevp[p] = pp[p * (Gm::IN_S / 2)];
-    }
 #pragma unroll
     for (int j = 0; j < RV; ++j) {
       const int gy = ty0 + yb + j;
@@ -437,17 +428,6 @@ __device__ __forceinline__ void blur_level_body(const ImagePlan* __restrict__ pl
         grow[0] = acc[j].x;
       }
       if constexpr (MODE == MODE_LEVEL) {
-        const int idx = (R & 1) + j;
-        const float4 pv = prevp[idx >> 1];
-        const float px = (idx & 1) ? pv.y : pv.x;
-        const float py = (idx & 1) ? pv.w : pv.z;
-        float* drow = dout + (long long)gy * O.pitch + gx;
-        const float dx0 = __fsub_rn(acc[j].x, px);
-        if (pair_ok) {
-          __stcs(reinterpret_cast<float2*>(drow), make_float2(dx0, __fsub_rn(acc[j].y, py)));
-        } else {
-          __stcs(drow, dx0);
-        }
         if (do_down && !(gy & 1)) {
           const OctaveDev& N = P.oct[octave + 1];
           const int dy = gy >> 1, dxn = gx >> 1;

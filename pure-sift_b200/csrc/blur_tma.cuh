@@ -17,8 +17,7 @@
 // overlap).  The horizontal pass takes two rows at a time: a thread's four
 // outputs of rows 2p and 2p + 1 as packed f32x2 pairs, each pair's operand
 // {x[2p][c], x[2p+1][c]} built from the two rows' 128-bit loads.  The vertical
-// pass runs from the intermediate and forms D = G[s] - G[s-1] with G[s-1] from
-// the stage.  Waits on the copies are bounded: on timeout the CTA records
+// pass runs from the intermediate.  Waits on the copies are bounded: on timeout the CTA records
 // kErrTimeout, waits (bounded) for its copies in flight and leaves.
 #pragma once
 #include <cuda.h>
@@ -191,7 +190,6 @@ __global__ void __launch_bounds__(kBlurThreads, TmaGeom<R>::MIN_CTAS)
     // Vertical pass: a column pair x RV rows per thread (as blur_level_kernel).
     {
       float* gout = O.g + (long long)level * O.plane_stride;
-      float* dout = O.d + (long long)(level - 1) * O.plane_stride;
       const bool do_down = level == down_level && octave + 1 < P.n_oct;
       const int x = 2 * lane;
       const int gx = tx0 + x;
@@ -211,21 +209,15 @@ __global__ void __launch_bounds__(kBlurThreads, TmaGeom<R>::MIN_CTAS)
         }
         if (gx >= w) continue;
         const bool pair_ok = gx + 1 < w;
-        // G[s-1] at (ty0 + yb + j, gx): stage row yb + j + R, column x + RP
-        const float* prev = s_in + (yb + R) * G::IN_W + x + G::RP;
 #pragma unroll
         for (int j = 0; j < RV; ++j) {
           const int gy = ty0 + yb + j;
           if (gy >= h) break;
-          const float2 pv = *reinterpret_cast<const float2*>(prev + j * G::IN_W);
           float* grow = gout + (long long)gy * O.pitch + gx;
-          float* drow = dout + (long long)gy * O.pitch + gx;
           if (pair_ok) {
             *reinterpret_cast<float2*>(grow) = acc[j];
-            __stcs(reinterpret_cast<float2*>(drow), make_float2(__fsub_rn(acc[j].x, pv.x), __fsub_rn(acc[j].y, pv.y)));
           } else {
             grow[0] = acc[j].x;
-            __stcs(drow, __fsub_rn(acc[j].x, pv.x));
           }
           if (do_down && !(gy & 1)) {
             const OctaveDev& N = P.oct[octave + 1];

@@ -27,8 +27,10 @@ cudaError_t launch_blur(int mode, const float* taps_host, int radius, const Imag
                         int level, int down_level, int max_h, int max_w, cudaStream_t st, int variant = 0,
                         bool fused = false, const TileMap* tiles = nullptr, const ImagePlan* h_plans = nullptr,
                         uint32_t* err = nullptr);
-cudaError_t launch_extrema_mark(const ImagePlan* plans, int n, int octave, int max_h, const ExtremaParams& prm,
-                                cudaStream_t st);
+cudaError_t launch_extrema_mark(const ImagePlan* plans, int n, int octave, int max_h, int max_w,
+                                const ExtremaParams& prm, cudaStream_t st);
+cudaError_t launch_dog_plane(const float* lower, const float* upper, long long pitch, int h, int w, float* out,
+                             cudaStream_t st);
 cudaError_t launch_row_scan(const ImagePlan* plans, int n, uint32_t kp_cap, uint32_t* err, cudaStream_t st);
 cudaError_t launch_extrema_emit(const ImagePlan* plans, int n, int octave, int max_h, const ExtremaParams& prm,
                                 uint32_t kp_cap, cudaStream_t st);
@@ -173,7 +175,7 @@ psift_status build_job(psift_ctx* ctx, const std::vector<ImageDesc>& imgs, const
     int rows = 0;
     for (int o = 0; o < job.n_oct[i]; ++o) {
       const HostOctave& O = job.oct[(size_t)i * kMaxOctaves + o];
-      total += align_up(plane_bytes(O) * (2 * S + 5), 256);
+      total += align_up(plane_bytes(O) * (S + 3), 256);
       total += align_up(sizeof(uint32_t) * (size_t)S * O.h * ((O.w + 31) / 32), 256);
       rows += S * O.h;
     }
@@ -207,9 +209,7 @@ psift_status build_job(psift_ctx* ctx, const std::vector<ImageDesc>& imgs, const
       O.w = H.w;
       O.pitch = H.pitch;
       O.plane_stride = H.pitch * H.h;
-      float* planes = (float*)arena_alloc(ctx, plane_bytes(H) * (2 * S + 5));
-      O.g = planes;
-      O.d = planes + O.plane_stride * (S + 3);
+      O.g = (float*)arena_alloc(ctx, plane_bytes(H) * (S + 3));
       O.words = (H.w + 31) / 32;
       O.masks = (uint32_t*)arena_alloc(ctx, sizeof(uint32_t) * (size_t)S * H.h * O.words);
       O.row_base = row_base;
@@ -353,7 +353,7 @@ psift_status launch_detect(psift_ctx* ctx, DetectJob& job, const psift_sift_conf
       }
     }
     StageScope sc_x(ctx, STAGE_EXTREMA, st);
-    cudaError_t e = launch_extrema_mark(job.d_plans, n, o, mh, xp, st);
+    cudaError_t e = launch_extrema_mark(job.d_plans, n, o, mh, mw, xp, st);
     ctx->launches++;
     if (e != cudaSuccess) return cuda_error(ctx, e, "extrema_mark");
   }
@@ -1143,7 +1143,9 @@ psift_status psift_build_pyramid(psift_ctx* ctx, const float* image, uint32_t h,
   void* extra = nullptr;
   psift_sift_config c = *cfg;
   c.max_features = 0;
-  st = build_job(ctx, imgs, c, job, img_bytes, &extra);
+  // behind the image: one DoG slice at a time on its way to the caller
+  const size_t dog_bytes = sizeof(float) * (size_t)oct[0].h * oct[0].w;
+  st = build_job(ctx, imgs, c, job, align_up(img_bytes, 256) + dog_bytes, &extra);
   if (st != PSIFT_OK) return st;
   job.plans[0].src = extra;
   PSIFT_CUDA_TRY(ctx, cudaMemcpy2DAsync(extra, sizeof(float) * w, image, sizeof(float) * stride, sizeof(float) * w, h,
@@ -1151,14 +1153,20 @@ psift_status psift_build_pyramid(psift_ctx* ctx, const float* image, uint32_t h,
   st = launch_pyramid_only(ctx, job, c);
   if (st != PSIFT_OK) return st;
   float* dst = planes;
+  float* dog = (float*)((char*)extra + align_up(img_bytes, 256));
   for (int o = 0; o < no; ++o) {
     const OctaveDev& O = job.plans[0].oct[o];
     const size_t hw = (size_t)O.h * O.w;
-    for (int i = 0; i < 2 * S + 5; ++i) {
-      const float* src = i < S + 3 ? O.g + (size_t)i * O.plane_stride : O.d + (size_t)(i - S - 3) * O.plane_stride;
-      PSIFT_CUDA_TRY(ctx, cudaMemcpy2DAsync(dst, sizeof(float) * O.w, src, sizeof(float) * O.pitch,
-                                            sizeof(float) * O.w, O.h, cudaMemcpyDeviceToHost, ctx->stream));
-      dst += hw;
+    for (int i = 0; i < S + 3; ++i, dst += hw)
+      PSIFT_CUDA_TRY(ctx, cudaMemcpy2DAsync(dst, sizeof(float) * O.w, O.g + (size_t)i * O.plane_stride,
+                                            sizeof(float) * O.pitch, sizeof(float) * O.w, O.h,
+                                            cudaMemcpyDeviceToHost, ctx->stream));
+    for (int i = 0; i < S + 2; ++i, dst += hw) {
+      const float* lower = O.g + (size_t)i * O.plane_stride;
+      const cudaError_t e = launch_dog_plane(lower, lower + O.plane_stride, O.pitch, O.h, O.w, dog, ctx->stream);
+      ctx->launches++;
+      if (e != cudaSuccess) return cuda_error(ctx, e, "dog_plane");
+      PSIFT_CUDA_TRY(ctx, cudaMemcpyAsync(dst, dog, sizeof(float) * hw, cudaMemcpyDeviceToHost, ctx->stream));
     }
   }
   PSIFT_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
@@ -1358,9 +1366,8 @@ bool carve_noalloc_job(FixedCarver& cv, const ImageDesc& img, const psift_sift_c
     O.w = H.w;
     O.pitch = H.pitch;
     O.plane_stride = H.pitch * H.h;
-    float* planes = (float*)cv.take(plane_bytes(H) * (2 * S + 5));
-    O.g = planes;
-    O.d = planes ? planes + O.plane_stride * (S + 3) : nullptr;
+    // the documented limit counts S + 2 more planes per octave than the S + 3 used
+    O.g = (float*)cv.take(plane_bytes(H) * (2 * S + 5));
     O.words = (H.w + 31) / 32;
     O.masks = (uint32_t*)cv.take(sizeof(uint32_t) * (size_t)S * H.h * O.words);
     O.row_base = row_base;

@@ -2,8 +2,10 @@
 //
 // HBM layout per image (all fp32 planes row-major, pitch = width rounded up to
 // 32 elements so every row starts on a 128-byte boundary):
-//   octave o: G[0..S+2] (S+3 Gaussian levels), D[0..S+1] (S+2 DoG slices),
+//   octave o: G[0..S+2] (S+3 Gaussian levels),
 //             extremum bitmask  [S][h][words]  (bit x%32 of word x/32),
+//             (the DoG slices D[i] = G[i+1] - G[i] are not stored: one rounded
+//             subtraction where they are read, see extrema.cu)
 //   rows:     per (octave, slice, row) keypoint counts and exclusive offsets,
 //   keypoints (capacity kp_cap) in the reference's (octave, slice, row, column) order,
 //   selected keypoints (top max_features by |response|, stable), 1..4
@@ -23,7 +25,6 @@ struct OctaveDev {
   long long pitch;         // elements
   long long plane_stride;  // elements between consecutive planes
   float* g;                // S+3 planes
-  float* d;                // S+2 planes
   uint32_t* masks;         // S * h * words
   int words;               // ceil(w / 32)
   int row_base;            // first row index of this octave in the image's row arrays

@@ -20,26 +20,44 @@
 
 namespace psift {
 
+// The 3x3x3 DoG values around pixel (x, y) of slice s, each the rounded difference
+// D[i] = G[i+1] - G[i] the pyramid defines (build_scale_space_pyramid_with_options,
+// src/pipeline.rs:550-638), formed here from the four Gaussian planes it spans
+// instead of being stored: the blur then writes one plane per level, not two
+// (20 of 64 bytes per octave pixel at 3 scales).  Entries are row-major, [4] the centre.
+struct Dog27 {
+  float p[9], c[9], n[9];
+};
+
+// g: G[s-1] at (x, y); every load is issued before the first use.
+__device__ __forceinline__ void load_dog27(const float* __restrict__ g, long long ps, long long pitch, Dog27& d) {
+  float v[4][9];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) v[i][3 * r + k] = __ldg(g + i * ps + (r - 1) * pitch + (k - 1));
+#pragma unroll
+  for (int k = 0; k < 9; ++k) {
+    d.p[k] = v[1][k] - v[0][k];
+    d.c[k] = v[2][k] - v[1][k];
+    d.n[k] = v[3][k] - v[2][k];
+  }
+}
+
 // refine_extremum_3d (src/pipeline.rs:697-770).
-__device__ __forceinline__ void refine3d(const float* __restrict__ p, const float* __restrict__ c,
-                                         const float* __restrict__ n, long long pitch, int x, float& ox_o,
-                                         float& oy_o, float& os_o, float& interp_o) {
-  const float* c_prev = c - pitch;
-  const float* c_next = c + pitch;
-  const float* p_prev = p - pitch;
-  const float* p_next = p + pitch;
-  const float* n_prev = n - pitch;
-  const float* n_next = n + pitch;
-  const float center = c[x];
-  const float gx = 0.5f * (c[x + 1] - c[x - 1]);
-  const float gy = 0.5f * (c_next[x] - c_prev[x]);
-  const float gs = 0.5f * (n[x] - p[x]);
-  const float dxx = c[x + 1] - 2.0f * center + c[x - 1];
-  const float dyy = c_next[x] - 2.0f * center + c_prev[x];
-  const float dss = n[x] - 2.0f * center + p[x];
-  const float dxy = 0.25f * ((c_next[x + 1] - c_next[x - 1]) - (c_prev[x + 1] - c_prev[x - 1]));
-  const float dxs = 0.25f * ((n[x + 1] - n[x - 1]) - (p[x + 1] - p[x - 1]));
-  const float dys = 0.25f * ((n_next[x] - n_prev[x]) - (p_next[x] - p_prev[x]));
+__device__ __forceinline__ void refine3d(const Dog27& d, float& ox_o, float& oy_o, float& os_o, float& interp_o) {
+  const float center = d.c[4];
+  const float gx = 0.5f * (d.c[5] - d.c[3]);
+  const float gy = 0.5f * (d.c[7] - d.c[1]);
+  const float gs = 0.5f * (d.n[4] - d.p[4]);
+  const float dxx = d.c[5] - 2.0f * center + d.c[3];
+  const float dyy = d.c[7] - 2.0f * center + d.c[1];
+  const float dss = d.n[4] - 2.0f * center + d.p[4];
+  const float dxy = 0.25f * ((d.c[8] - d.c[6]) - (d.c[2] - d.c[0]));
+  const float dxs = 0.25f * ((d.n[5] - d.n[3]) - (d.p[5] - d.p[3]));
+  const float dys = 0.25f * ((d.n[7] - d.n[1]) - (d.p[7] - d.p[1]));
   const float c00 = dyy * dss - dys * dys;
   const float c01 = dys * dxs - dxy * dss;
   const float c02 = dxy * dys - dyy * dxs;
@@ -81,167 +99,172 @@ __device__ __forceinline__ void refine3d(const float* __restrict__ p, const floa
   interp_o = center;
 }
 
-// Full acceptance test for pixel (x, y) of slice `c` (rows already offset to y).
-// The reference's comparison chain (is_greater/less_than_patch3x3 over the
-// current, previous and next slices) is evaluated on loads issued together: the
-// 8 same-slice neighbours first, then, only if they pass, the 18 of the other
-// two slices.  Short-circuiting does not change the outcome (all must hold).
-__device__ __forceinline__ bool accept_pixel(const float* __restrict__ p, const float* __restrict__ c,
-                                             const float* __restrict__ n, long long pitch, int x, float thr) {
-  const float v = c[x];
+// Full acceptance test for the pixel whose neighbourhood is d: the reference's
+// comparison chain (is_greater/less_than_patch3x3 over the current, previous and
+// next slices), its edge test and its refinement.  Short-circuiting does not
+// change the outcome (all must hold).
+__device__ __forceinline__ bool accept_pixel(const Dog27& d, float thr) {
+  const float v = d.c[4];
   if (fabsf(v) <= thr) return false;
-  // All 26 neighbours are loaded before the first test: a warp's candidates are
-  // tested together, so one of them passing the same-slice test would otherwise
-  // make the whole warp wait for a second round of loads.
-  const float* ca = c - pitch;
-  const float* cb = c + pitch;
-  float nb[9];
-  nb[0] = ca[x - 1]; nb[1] = ca[x]; nb[2] = ca[x + 1];
-  nb[3] = c[x - 1];  nb[4] = c[x + 1];
-  nb[5] = cb[x - 1]; nb[6] = cb[x]; nb[7] = cb[x + 1];
-  float pn[18];
-  {
-    const float* pa = p - pitch;
-    const float* pb = p + pitch;
-    const float* na = n - pitch;
-    const float* nbp = n + pitch;
-    pn[0] = pa[x - 1];  pn[1] = pa[x];  pn[2] = pa[x + 1];
-    pn[3] = p[x - 1];   pn[4] = p[x];   pn[5] = p[x + 1];
-    pn[6] = pb[x - 1];  pn[7] = pb[x];  pn[8] = pb[x + 1];
-    pn[9] = na[x - 1];  pn[10] = na[x]; pn[11] = na[x + 1];
-    pn[12] = n[x - 1];  pn[13] = n[x];  pn[14] = n[x + 1];
-    pn[15] = nbp[x - 1]; pn[16] = nbp[x]; pn[17] = nbp[x + 1];
-  }
   const bool pos = v > 0.0f;
   bool ext = true;
 #pragma unroll
-  for (int k = 0; k < 8; ++k) ext = ext && (pos ? v > nb[k] : v < nb[k]);
-  if (!ext) return false;
-#pragma unroll
-  for (int k = 0; k < 18; ++k) ext = ext && (pos ? v > pn[k] : v < pn[k]);
+  for (int k = 0; k < 9; ++k) {
+    if (k != 4) ext = ext && (pos ? v > d.c[k] : v < d.c[k]);
+    ext = ext && (pos ? v > d.p[k] : v < d.p[k]);
+    ext = ext && (pos ? v > d.n[k] : v < d.n[k]);
+  }
   if (!ext) return false;
   // passes_hessian_edge_test (src/pipeline.rs:664-687)
   {
-    const float dxx = nb[4] - 2.0f * v + nb[3];
-    const float dyy = nb[6] - 2.0f * v + nb[1];
-    const float dxy = 0.25f * ((nb[7] - nb[5]) - (nb[2] - nb[0]));
+    const float dxx = d.c[5] - 2.0f * v + d.c[3];
+    const float dyy = d.c[7] - 2.0f * v + d.c[1];
+    const float dxy = 0.25f * ((d.c[8] - d.c[6]) - (d.c[2] - d.c[0]));
     const float trace = dxx + dyy;
     const float det = dxx * dyy - dxy * dxy;
     const float ratio = (11.0f * 11.0f) / 10.0f;
     if (!(det > 1e-9f && (trace * trace) < ratio * det)) return false;
   }
   float ox, oy, os, interp;
-  refine3d(p, c, n, pitch, x, ox, oy, os, interp);
+  refine3d(d, ox, oy, os, interp);
   return fabsf(interp) > thr;
 }
 
-// Grid (ceil(max_h / 4), scales, images), 128 threads: one warp per (row,
-// slice, image), no block-wide barriers.  The warp walks its row in 256-pixel
-// spans (a lane reads 8 pixels as two 128-bit loads, 128 pixels apart; the
-// next span's loads are issued before the current span is processed); a span is
-// exactly 8 mask words.
-//   A. streaming: pixels with |v| > threshold (the reference's first test, a
-//      small fraction of the row) become candidates; a span without any writes
-//      zero words;
-//   B. otherwise the candidates are compacted into the warp's shared-memory
-//      queue and the warp runs the full 26-neighbour / Hessian / refinement
-//      test on them only, setting bits of the span's 8 mask words.
+// 128 threads per CTA; WPR warps share a row (all S slices), 4 / WPR rows per CTA.
+// A warp walks every WPR-th 128-pixel span of its row (a lane reads 4 pixels of
+// each of the planes G[1..S+1] as 128-bit loads; the next span's loads are issued
+// before the current span is processed).
+//   A. streaming: a pixel of slice s stays a candidate if its D is above the
+//      threshold and above every neighbour at hand, or below the negated threshold
+//      and below every neighbour at hand: left and right (inside the span) and
+//      slices s - 1, s + 1 where they are among the loaded ones.  Each of these
+//      comparisons is part of the full test, so nothing is lost, and the survivors
+//      are a few per row instead of every pixel of a blob.
+//   B. survivors queue up in shared memory and take the full 26-neighbour /
+//      Hessian / refinement test 32 at a time; accepted ones set their bit of the
+//      row's mask words (zeroed first).
+// Bound by HBM latency and the comparisons' issue: 4 (S + 1) bytes per pixel read
+// once, 57 us for two 3840 x 2160 octaves at 3 scales (4.7 TB/s, 78 us with a warp
+// per row: four warps per row keep the last wave of a launch short).
 constexpr int kMarkWarps = 4;
-constexpr int kMarkSpan = 256;  // pixels per warp step
+constexpr int kMarkSpan = 128;  // pixels per warp step
 
-__device__ __forceinline__ void mark_load_span(const float* __restrict__ Dc, int xb, int lane, int w, float4 (&v)[2]) {
+template <int S>
+__device__ __forceinline__ void mark_load_span(const float* __restrict__ g1, long long ps, int x0, int w,
+                                               float4 (&v)[S + 1]) {
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int x0 = xb + h * 128 + 4 * lane;
+  for (int i = 0; i <= S; ++i) {
+    const float* g = g1 + i * ps + x0;
     if (x0 + 3 < w) {
-      v[h] = *reinterpret_cast<const float4*>(Dc + x0);
+      v[i] = __ldg(reinterpret_cast<const float4*>(g));
     } else {
-      v[h] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      if (x0 + 0 < w) v[h].x = Dc[x0 + 0];
-      if (x0 + 1 < w) v[h].y = Dc[x0 + 1];
-      if (x0 + 2 < w) v[h].z = Dc[x0 + 2];
+      v[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (x0 + 0 < w) v[i].x = g[0];
+      if (x0 + 1 < w) v[i].y = g[1];
+      if (x0 + 2 < w) v[i].z = g[2];
     }
   }
 }
 
+template <int S, int WPR>
 __global__ void __launch_bounds__(kMarkWarps * 32) extrema_mark_kernel(const ImagePlan* __restrict__ plans,
                                                                        int octave, ExtremaParams prm) {
-  const ImagePlan& P = plans[blockIdx.z];
+  constexpr int ROWS = kMarkWarps / WPR;
+  __shared__ uint32_t s_q[kMarkWarps][31 + S * kMarkSpan];  // (s - 1) << 16 | x
+  __shared__ uint32_t s_cnt[ROWS][S];
+  const ImagePlan& P = plans[blockIdx.y];
   if (octave >= P.n_oct) return;
   const OctaveDev& O = P.oct[octave];
+  if ((int)blockIdx.x * ROWS >= O.h) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int y = blockIdx.y * kMarkWarps + warp;
-  if (y >= O.h) return;
-  const int s = blockIdx.x + 1;  // slices fastest: the three slices of a row band share D rows in L2
-  const long long ps = O.plane_stride;
-  const float* Dp = O.d + (long long)(s - 1) * ps + (long long)y * O.pitch;
-  const float* Dc = O.d + (long long)s * ps + (long long)y * O.pitch;
-  const float* Dn = O.d + (long long)(s + 1) * ps + (long long)y * O.pitch;
-  uint32_t* mrow = O.masks + ((long long)(s - 1) * O.h + y) * O.words;
-  const float thr = prm.threshold;
-  const bool row_ok = y >= 1 && y < O.h - 1;
-  const int w = O.w;
-  const int span_end = O.words * 32;
+  const int row = warp / WPR, part = warp % WPR;
+  const int y = blockIdx.x * ROWS + row;
+  const long long ps = O.plane_stride, pitch = O.pitch;
+  const int w = O.w, words = O.words;
+  const long long slice_words = (long long)O.h * words;
+  uint32_t* mrow = O.masks + (long long)y * words;  // slice 1's; slice s: + (s - 1) * slice_words
+  const int tid = threadIdx.x % (32 * WPR);         // thread of the row
+  if (tid < S) s_cnt[row][tid] = 0;
+  if (y < O.h)
+    for (int s = 0; s < S; ++s)
+      for (int i = tid; i < words; i += 32 * WPR) mrow[s * slice_words + i] = 0;
+  __syncthreads();  // the zeroed words and counts before the bits set in them
+  if (y >= 1 && y < O.h - 1) {
+    const float* g0 = O.g + (long long)y * pitch;  // G[0], row y
+    const float* g1 = g0 + ps;
+    const float thr = prm.threshold;
+    const float none = __int_as_float(0x7fffffff);  // NaN: ignored by fmaxf / fminf
+    uint32_t* q = s_q[warp];
+    int queued = 0;
+    auto test = [&](int i) {
+      const uint32_t e = q[i];
+      const int s = (int)(e >> 16), x = (int)(e & 0xFFFFu);
+      if (x < 1 || x >= w - 1) return;
+      Dog27 d;
+      load_dog27(g0 + s * ps + x, ps, pitch, d);  // G[s-1] of slice s (e holds s - 1)
+      if (accept_pixel(d, thr)) {
+        atomicOr(mrow + s * slice_words + (x >> 5), 1u << (x & 31));
+        atomicAdd(&s_cnt[row][s], 1u);
+      }
+    };
 
-  __shared__ uint16_t s_q[kMarkWarps][kMarkSpan];
-  __shared__ uint32_t s_mask[kMarkWarps][kMarkSpan / 32];
-  uint16_t* q = s_q[warp];
-  uint32_t* wm = s_mask[warp];
-  uint32_t cnt = 0;
-
-  float4 cur[2], nxt[2];
-  if (row_ok) mark_load_span(Dc, 0, lane, w, cur);
-  for (int xb = 0; xb < span_end; xb += kMarkSpan) {
-    if (row_ok && xb + kMarkSpan < span_end) mark_load_span(Dc, xb + kMarkSpan, lane, w, nxt);
-    uint32_t m = 0;  // bit 4h + i: pixel xb + 128 h + 4 lane + i
-    if (row_ok) {
+    float4 cur[S + 1], nxt[S + 1];
+    mark_load_span<S>(g1, ps, part * kMarkSpan + 4 * lane, w, cur);
+    for (int xb = part * kMarkSpan; xb < w; xb += WPR * kMarkSpan) {
+      if (xb + WPR * kMarkSpan < w) mark_load_span<S>(g1, ps, xb + WPR * kMarkSpan + 4 * lane, w, nxt);
+      float D[S][4];
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const float e[4] = {cur[h].x, cur[h].y, cur[h].z, cur[h].w};
+      for (int s = 0; s < S; ++s) {
+        D[s][0] = cur[s + 1].x - cur[s].x;
+        D[s][1] = cur[s + 1].y - cur[s].y;
+        D[s][2] = cur[s + 1].z - cur[s].z;
+        D[s][3] = cur[s + 1].w - cur[s].w;
+      }
+      unsigned long long m = 0;  // bit 4 (s - 1) + i: pixel xb + 4 lane + i of slice s
+#pragma unroll
+      for (int s = 0; s < S; ++s) {
+        float left = __shfl_up_sync(0xffffffffu, D[s][3], 1), right = __shfl_down_sync(0xffffffffu, D[s][0], 1);
+        if (lane == 0) left = none;
+        if (lane == 31) right = none;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const int x = xb + h * 128 + 4 * lane + i;
-          // the reference's first rejection is |v| <= threshold (NaN continues)
-          if (x >= 1 && x < w - 1 && !(fabsf(e[i]) <= thr)) m |= 1u << (4 * h + i);
+          const float v = D[s][i];
+          const float l = i > 0 ? D[s][i > 0 ? i - 1 : 0] : left, r = i < 3 ? D[s][i < 3 ? i + 1 : 3] : right;
+          float hi = fmaxf(fmaxf(thr, l), r), lo = fminf(fminf(-thr, l), r);
+          if (s > 0) hi = fmaxf(hi, D[s > 0 ? s - 1 : 0][i]), lo = fminf(lo, D[s > 0 ? s - 1 : 0][i]);
+          if (s + 1 < S) hi = fmaxf(hi, D[s + 1 < S ? s + 1 : s][i]), lo = fminf(lo, D[s + 1 < S ? s + 1 : s][i]);
+          if (v > hi || v < lo) m |= 1ull << (4 * s + i);
         }
       }
-    }
-    uint32_t word_bits = 0;  // lane < 8: mask word (xb >> 5) + lane
-    if (__any_sync(0xffffffffu, m != 0)) {
-      const uint32_t c = __popc(m);
-      uint32_t incl = c;
+      if (__any_sync(0xffffffffu, m != 0)) {
+        const int c = __popcll(m);
+        int incl = c;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += t;
+        for (int o = 1; o < 32; o <<= 1) {
+          const int t = __shfl_up_sync(0xffffffffu, incl, o);
+          if (lane >= o) incl += t;
+        }
+        int pos = queued + incl - c;
+        while (m) {
+          const int b = __ffsll((long long)m) - 1;
+          m &= m - 1;
+          q[pos++] = (uint32_t)(b >> 2) << 16 | (uint32_t)(xb + 4 * lane + (b & 3));
+        }
+        queued += __shfl_sync(0xffffffffu, incl, 31);
+        __syncwarp();
+        while (queued >= 32) {
+          queued -= 32;
+          test(queued + lane);
+        }
+        __syncwarp();
       }
-      const int total = (int)__shfl_sync(0xffffffffu, incl, 31);
-      uint32_t pos = incl - c;
 #pragma unroll
-      for (int b = 0; b < 8; ++b)
-        if (m & (1u << b)) q[pos++] = (uint16_t)((b >> 2) * 128 + 4 * lane + (b & 3));
-      if (lane < 8) wm[lane] = 0;
-      __syncwarp();
-      for (int i = lane; i < total; i += 32) {
-        const int off = q[i];
-        if (accept_pixel(Dp, Dc, Dn, O.pitch, xb + off, thr)) atomicOr(&wm[off >> 5], 1u << (off & 31));
-      }
-      __syncwarp();
-      if (lane < 8) word_bits = wm[lane];
-      __syncwarp();
+      for (int i = 0; i <= S; ++i) cur[i] = nxt[i];
     }
-    if (lane < 8) {
-      const int word = (xb >> 5) + lane;
-      if (word < O.words) {
-        mrow[word] = word_bits;
-        cnt += __popc(word_bits);
-      }
-    }
-    cur[0] = nxt[0];
-    cur[1] = nxt[1];
+    if (lane < queued) test(lane);
   }
-  cnt = __reduce_add_sync(0xffffffffu, cnt);
-  if (lane == 0) P.row_counts[O.row_base + (s - 1) * O.h + y] = cnt;
+  __syncthreads();
+  if (y < O.h && tid < S) P.row_counts[O.row_base + tid * O.h + y] = s_cnt[row][tid];
 }
 
 // Block-wide exclusive scan helper for 1024 threads; returns the block total.
@@ -307,9 +330,7 @@ __global__ void __launch_bounds__(256) extrema_emit_kernel(const ImagePlan* __re
   const int y = row_local - (s - 1) * O.h;
   uint32_t pos_base = P.row_offsets[r];
   const long long ps = O.plane_stride;
-  const float* Dp = O.d + (long long)(s - 1) * ps + (long long)y * O.pitch;
-  const float* Dc = O.d + (long long)s * ps + (long long)y * O.pitch;
-  const float* Dn = O.d + (long long)(s + 1) * ps + (long long)y * O.pitch;
+  const float* g = O.g + (long long)(s - 1) * ps + (long long)y * O.pitch;  // G[s-1], row y
   const uint32_t* mrow = O.masks + ((long long)(s - 1) * O.h + y) * O.words;
   const float mult = O.scale_factor;
   const float eff = prm.eff_scale[octave][s];
@@ -328,7 +349,9 @@ __global__ void __launch_bounds__(256) extrema_emit_kernel(const ImagePlan* __re
       word &= word - 1;
       const int x = (wb + lane) * 32 + b;
       float dx, dy, ds, interp;
-      refine3d(Dp, Dc, Dn, O.pitch, x, dx, dy, ds, interp);
+      Dog27 d;
+      load_dog27(g + x, ps, O.pitch, d);
+      refine3d(d, dx, dy, ds, interp);
       if (pos < kp_cap) {
         psift_keypoint kp;
         const float kds = (float)pow((double)prm.k, (double)ds);
@@ -439,10 +462,47 @@ __global__ void __launch_bounds__(1024) select_topk_kernel(const ImagePlan* __re
   if (threadIdx.x == 0) *P.sel_count = K;
 }
 
-cudaError_t launch_extrema_mark(const ImagePlan* plans, int n, int octave, int max_h, const ExtremaParams& prm,
-                                cudaStream_t st) {
-  dim3 grid(prm.scales, (max_h + kMarkWarps - 1) / kMarkWarps, n);
-  extrema_mark_kernel<<<grid, kMarkWarps * 32, 0, st>>>(plans, octave, prm);
+template <int S>
+static void launch_mark_s(const ImagePlan* plans, int n, int octave, int max_h, int max_w, const ExtremaParams& prm,
+                          cudaStream_t st) {
+  // at least two spans per warp of a row
+  if (max_w > 6 * kMarkSpan)
+    extrema_mark_kernel<S, 4><<<dim3(max_h, n), kMarkWarps * 32, 0, st>>>(plans, octave, prm);
+  else if (max_w > 3 * kMarkSpan)
+    extrema_mark_kernel<S, 2><<<dim3((max_h + 1) / 2, n), kMarkWarps * 32, 0, st>>>(plans, octave, prm);
+  else
+    extrema_mark_kernel<S, 1><<<dim3((max_h + 3) / 4, n), kMarkWarps * 32, 0, st>>>(plans, octave, prm);
+}
+
+cudaError_t launch_extrema_mark(const ImagePlan* plans, int n, int octave, int max_h, int max_w,
+                                const ExtremaParams& prm, cudaStream_t st) {
+  switch (prm.scales) {
+#define PSIFT_MARK(SS)                                              \
+  case SS:                                                          \
+    launch_mark_s<SS>(plans, n, octave, max_h, max_w, prm, st);     \
+    break;
+    PSIFT_MARK(3) PSIFT_MARK(4) PSIFT_MARK(5) PSIFT_MARK(6) PSIFT_MARK(7) PSIFT_MARK(8) PSIFT_MARK(9) PSIFT_MARK(10)
+#undef PSIFT_MARK
+    default:
+      return cudaErrorInvalidValue;  // scales is validated to 3..10
+  }
+  return cudaGetLastError();
+}
+
+// One stored DoG slice, G[i+1] - G[i] (psift_build_pyramid hands the slices to the caller).
+__global__ void dog_plane_kernel(const float* __restrict__ lower, const float* __restrict__ upper, long long pitch,
+                                 int h, int w, float* __restrict__ out) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)h * w;
+       i += (long long)gridDim.x * blockDim.x) {
+    const int y = (int)(i / w), x = (int)(i - (long long)y * w);
+    out[i] = upper[y * pitch + x] - lower[y * pitch + x];
+  }
+}
+
+cudaError_t launch_dog_plane(const float* lower, const float* upper, long long pitch, int h, int w, float* out,
+                             cudaStream_t st) {
+  const long long blocks = ((long long)h * w + 255) / 256;
+  dog_plane_kernel<<<(unsigned)(blocks < 148 * 32 ? blocks : 148 * 32), 256, 0, st>>>(lower, upper, pitch, h, w, out);
   return cudaGetLastError();
 }
 
