@@ -115,8 +115,9 @@ psift_status psift_ctx_enable_stage_timing(psift_ctx* ctx, int enable);
 
 /* Tile shapes, chosen by the library's autotuner.  No counterpart in the
  * reference.  Every choice computes identical results; only time differs.
- *  - PSIFT_TUNE_BLUR, index = radius 1..15: the level blur's kernel: outputs per
- *    thread 0: 4 columns x 8 rows (the default), 1: 8 x 8, 2: 4 x 4; 3: TMA
+ *  - PSIFT_TUNE_BLUR, index = radius 1..15: the level blur's kernel: 0 (the
+ *    default): a warp per 64-column strip for large launches, else 4 columns x 8
+ *    rows of outputs per thread; 1: 8 x 8, 2: 4 x 4 outputs per thread; 3: TMA
  *    tiles with persistent CTAs (batches of at most 64 images; larger ones use 0);
  *    4: 128-row tiles of 512 threads (4 x 8 outputs per thread).
  *    A batch of images of different sizes runs variant 0's shape (or 3) over a

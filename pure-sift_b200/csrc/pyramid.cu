@@ -7,8 +7,9 @@
 namespace psift {
 
 // Host entry: mode 0 = level blur (octave, level >= 1); modes 1..4 = octave-0 base.
-// variant (level blur only) picks the outputs per thread (0-2, see
-// blur_kernel.cuh), the TMA-tile kernel (3, blur_tma.cuh; needs the host copy
+// variant (level blur only) picks the default (0: strips for large launches,
+// blur_strip.cuh, else 4 x 8 outputs per thread), other outputs per thread (1, 2,
+// see blur_kernel.cuh), the TMA-tile kernel (3, blur_tma.cuh; needs the host copy
 // of the plans for its tensor maps) or 128 x 64 tiles of 512 threads (4: half
 // the horizontal pass's halo rows per output); every variant computes the same
 // values.  fused: the single-rounding blur
@@ -16,6 +17,12 @@ namespace psift {
 cudaError_t launch_blur_tma(int radius, bool fused, const ImagePlan* d_plans, const ImagePlan* h_plans, int n,
                             int octave, int level, int down_level, int zrev, const Taps2& taps, uint32_t* err,
                             cudaStream_t st);
+
+cudaError_t launch_blur_strip(int radius, bool fused, const ImagePlan* plans, const ImagePlan* h_plans, int n,
+                              int octave, int level, int down_level, int zrev, const Taps2& taps, int max_h,
+                              int max_w, cudaStream_t st);
+constexpr int kStripMaxR = 10;                    // largest radius of the strip kernel
+constexpr long long kStripMinPixels = 6000000;
 
 cudaError_t launch_blur(int mode, const float* taps_host, int radius, const ImagePlan* plans, int n, int octave,
                         int level, int down_level, int max_h, int max_w, cudaStream_t st, int variant, bool fused,
@@ -27,6 +34,21 @@ cudaError_t launch_blur(int mode, const float* taps_host, int radius, const Imag
   }
   t.one = make_float2(1.0f, 1.0f);
   const int zrev = (octave * 8 + level) & 1;
+  // Variant 0: strips from kStripMinPixels output pixels per launch, else tiles.  A
+  // strip's warp needs 6 to 10 us for its chunk however small the launch is, a tile
+  // CTA 5 to 7 us (640 x 480, R = 4 / 10: strips 8.4 / 13.2 us, tiles 7.4 / 11.6);
+  // two 1920 x 1080 planes take the same time either way (13.9 .. 30 against 15.2
+  // .. 24 us), one 3840 x 2160 plane 19.4 / 25 / 30 / 25 / 41 us as strips and 25.3
+  // / 28 / 31 / 35 / 41 as tiles.
+  if (mode == MODE_LEVEL && variant == 0 && radius <= kStripMaxR) {
+    long long pixels = 0;
+    for (int i = 0; i < n; ++i) {
+      if (!h_plans) pixels += (long long)max_h * max_w;
+      else if (octave < h_plans[i].n_oct) pixels += (long long)h_plans[i].oct[octave].h * h_plans[i].oct[octave].w;
+    }
+    if (pixels >= kStripMinPixels)
+      return launch_blur_strip(radius, fused, plans, h_plans, n, octave, level, down_level, zrev, t, max_h, max_w, st);
+  }
   // variant 3: TMA tiles, persistent CTAs (blur_tma.cuh), either rounding
   if (mode == MODE_LEVEL && variant == 3)
     return launch_blur_tma(radius, fused, plans, h_plans, n, octave, level, down_level, zrev, t, err, st);
