@@ -13,7 +13,7 @@
 
 namespace psift {
 
-cudaError_t launch_ransac(const RansacJob* jobs, int n_jobs, cudaStream_t st);
+cudaError_t launch_ransac(const RansacJob* jobs, int n_jobs, int num_sms, cudaStream_t st);
 
 namespace {
 constexpr uint64_t kSimSeed = 0xD1B54A32D192ED03ull;   // DEFAULT_SIMILARITY_RANSAC_SEED, src/pipeline.rs:172
@@ -68,7 +68,7 @@ psift_status run_batch(psift_ctx* ctx, const psift_ransac_job* jobs, int n, cons
   }
   PSIFT_CUDA_TRY(ctx, cudaMemcpyAsync(d_jobs, hj.data(), sizeof(RansacJob) * n, cudaMemcpyHostToDevice, ctx->stream));
   StageScope sc(ctx, STAGE_RANSAC);
-  cudaError_t e = launch_ransac(d_jobs, n, ctx->stream);
+  cudaError_t e = launch_ransac(d_jobs, n, ctx->num_sms, ctx->stream);
   ctx->launches++;
   if (e != cudaSuccess) return cuda_error(ctx, e, "ransac");
   return PSIFT_OK;
