@@ -14,9 +14,10 @@
 //
 // The reference's loop is replayed exactly: its draws are resolved in parallel
 // (ransac_common.cuh), thread 0 walks them to form the same 8-index samples
-// (distinct indices, at most 32 attempts), 64 samples are fitted at a time (one
-// quad of lanes each, the reference's f64 operations in its order), each warp counts
-// the inliers of 8 of them, and thread 0 takes every decision in order: count,
+// (distinct indices, at most 32 attempts), a batch of samples (a quarter of the
+// CTA's threads) is fitted at a time (one quad of lanes each, the reference's f64
+// operations in its order), each warp counts the inliers of 8 of them, and thread 0
+// takes every decision in order: count,
 // the tie-break on the truncated error sum (the reference's sequential sum over
 // the matches, evaluated only when a tie needs it), the adaptive iteration
 // budget, then up to two LO refits over the ordered inlier list (the 45 entries
@@ -34,10 +35,6 @@
 namespace psift {
 namespace {
 
-constexpr int kFThreads = 256;
-constexpr int kFB = 64;      // hypotheses per batch
-constexpr int kFWin = 2048;  // resolved draws per window (>= 32 per iteration)
-
 struct FundJob {
   const psift_match* m;
   int n;
@@ -47,33 +44,12 @@ struct FundJob {
   double* cdf;    // n
   double* terms;  // n
   double* pts;    // 4 per match: the ordered inlier list's coordinates, gathered
+  float4* xy;     // (query x, query y, target x, target y) per match
   uint8_t* mask;
   double* f9;
   int* has_f;
   int* count;
   int* iters;
-};
-
-struct FShared {
-  double F[kFB][9];
-  int samp[kFB][8];
-  int sok[kFB], fok[kFB], cnt[kFB], sdup[kFB];
-  int draws[kFWin];
-  double best[9], cand[9];
-  double best_err;
-  int best_err_known, best_count, have, max_iters, iter;
-  int nb, refill;
-  long long tpos, wb;
-  // decision flags of the replay
-  int act;
-  double ev_err;
-  int ev_cnt;
-  // LO refit
-  int list_n, fit_ok;
-  double sums[6];  // qx qy tx ty (sums), then mean distances q, t
-  double ata[9][9];
-  uint32_t red_u[kFThreads / 32];
-  int scan[kFThreads / 32];
 };
 
 // ------------------------------------------------------------ 3x3 / vector helpers
@@ -510,8 +486,8 @@ __device__ bool quad_fit8(const psift_match* __restrict__ m, const int* idx, dou
   return finish_from_eigen(A, V, norm_T(qs, qcx, qcy), norm_T(ts, tcx, tcy), out);
 }
 
-__device__ __forceinline__ double sampson(const double* f, const psift_match& a) {
-  const double x1 = (double)a.query_x, y1 = (double)a.query_y, x2 = (double)a.target_x, y2 = (double)a.target_y;
+__device__ __forceinline__ double sampson(const double* f, const float4 a) {
+  const double x1 = (double)a.x, y1 = (double)a.y, x2 = (double)a.z, y2 = (double)a.w;
   const double a0 = f[0] * x1 + f[1] * y1 + f[2];
   const double a1 = f[3] * x1 + f[4] * y1 + f[5];
   const double a2 = f[6] * x1 + f[7] * y1 + f[8];
@@ -528,8 +504,7 @@ __device__ __forceinline__ double sampson(const double* f, const psift_match& a)
 // ee <= p (1 - 2^-50) and round(ee / den) > tsq when ee >= p (1 + 2^-50) (the
 // margins cover the roundings of p, of the margin product and of the quotient);
 // in between, and for NaN, the reference's quotient decides.
-__device__ __forceinline__ bool sampson_in(const double* f, const psift_match& a, double tsq) {
-  const double x1 = (double)a.query_x, y1 = (double)a.query_y, x2 = (double)a.target_x, y2 = (double)a.target_y;
+__device__ __forceinline__ bool sampson_in(const double* f, double x1, double y1, double x2, double y2, double tsq) {
   const double a0 = f[0] * x1 + f[1] * y1 + f[2];
   const double a1 = f[3] * x1 + f[4] * y1 + f[5];
   const double a2 = f[6] * x1 + f[7] * y1 + f[8];
@@ -623,8 +598,43 @@ __device__ int cubic_roots(double c3, double c2, double c1, double c0, double* r
   return k;
 }
 
+// A CTA's threads, by the number of match sets of a launch: 256 (two CTAs per SM),
+// or, up to one set per SM, 512: twice the samples fitted and counted per batch in
+// little more time (the fits are latency-bound chains).  48 sets of 2000 to 8000
+// matches, outliers 10 to 60 %: 13.9 against 24.5 ms, with the matches packed to 16
+// bytes and counts that stop once they cannot reach the incumbent's.
+template <int THREADS>
+struct FundCta {
+static constexpr int kFThreads = THREADS;
+static constexpr int kFB = THREADS / 4;  // hypotheses per batch, a quad of lanes each
+static constexpr int kFWin = 32 * kFB;   // resolved draws per window (>= 32 per iteration)
+static constexpr int kPass = 2;          // hypotheses a warp counts per pass over the matches
+static constexpr int kCheck = 16;        // matches per lane between checks for an early end
+
+struct FShared {
+  double F[kFB][9];
+  int samp[kFB][8];
+  int sok[kFB], fok[kFB], cnt[kFB], sdup[kFB];
+  int draws[kFWin];
+  double best[9], cand[9];
+  double best_err;
+  int best_err_known, best_count, have, max_iters, iter;
+  int nb, refill;
+  long long tpos, wb;
+  // decision flags of the replay
+  int act;
+  double ev_err;
+  int ev_cnt;
+  // LO refit
+  int list_n, fit_ok;
+  double sums[6];  // qx qy tx ty (sums), then mean distances q, t
+  double ata[9][9];
+  uint32_t red_u[kFThreads / 32];
+  int scan[kFThreads / 32];
+};
+
 // ------------------------------------------------------------ block helpers
-__device__ int block_sum(int v, FShared& S) {
+static __device__ int block_sum(int v, FShared& S) {
   for (int o = 16; o >= 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   __syncthreads();
   if ((threadIdx.x & 31) == 0) S.red_u[threadIdx.x >> 5] = (uint32_t)v;
@@ -637,8 +647,8 @@ __device__ int block_sum(int v, FShared& S) {
 
 // Sequential sum of v[0..n) in order, the loads issued kSeqAhead at a time ahead
 // of the dependent adds (one thread).
-constexpr int kSeqAhead = 16;
-__device__ double seq_sum(const double* __restrict__ v, int n) {
+static constexpr int kSeqAhead = 16;
+static __device__ double seq_sum(const double* __restrict__ v, int n) {
   double acc = 0.0;
   int i = 0;
   for (; i + kSeqAhead <= n; i += kSeqAhead) {
@@ -654,10 +664,10 @@ __device__ double seq_sum(const double* __restrict__ v, int n) {
 
 // evaluate_fundamental_hypothesis of f (shared): count (whole CTA) and the
 // truncated error sum in match order (terms in parallel, summed by thread 0).
-__device__ void evaluate(const FundJob& J, FShared& S, const double* f, int& count, double& err) {
+static __device__ void evaluate(const FundJob& J, FShared& S, const double* f, int& count, double& err) {
   int c = 0;
   for (int i = threadIdx.x; i < J.n; i += kFThreads) {
-    const double d2 = sampson(f, J.m[i]);
+    const double d2 = sampson(f, J.xy[i]);
     const bool in = d2 <= J.tsq;
     c += in;
     J.terms[i] = in ? d2 : J.tsq;
@@ -671,12 +681,12 @@ __device__ void evaluate(const FundJob& J, FShared& S, const double* f, int& cou
 
 // Ordered inlier list of S.best, its coordinates gathered into J.pts; returns its
 // length (whole CTA).
-__device__ int collect(const FundJob& J, FShared& S) {
+static __device__ int collect(const FundJob& J, FShared& S) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int base = 0;
   for (int b0 = 0; b0 < J.n; b0 += kFThreads) {
     const int i = b0 + threadIdx.x;
-    const bool in = i < J.n && sampson(S.best, J.m[i]) <= J.tsq;
+    const bool in = i < J.n && sampson(S.best, J.xy[i]) <= J.tsq;
     const uint32_t bal = __ballot_sync(0xffffffffu, in);
     if (lane == 0) S.scan[warp] = __popc(bal);
     __syncthreads();
@@ -684,9 +694,8 @@ __device__ int collect(const FundJob& J, FShared& S) {
     for (int w = 0; w < warp; ++w) off += S.scan[w];
     if (in) {
       const int pos = off + __popc(bal & ((1u << lane) - 1u));
-      const psift_match& a = J.m[i];
-      reinterpret_cast<double4*>(J.pts)[pos] =
-          make_double4((double)a.query_x, (double)a.query_y, (double)a.target_x, (double)a.target_y);
+      const float4 a = J.xy[i];
+      reinterpret_cast<double4*>(J.pts)[pos] = make_double4((double)a.x, (double)a.y, (double)a.z, (double)a.w);
     }
     int tot = 0;
     for (int w = 0; w < kFThreads / 32; ++w) tot += S.scan[w];
@@ -699,7 +708,7 @@ __device__ int collect(const FundJob& J, FShared& S) {
 // fit_fundamental_8point over the gathered inliers J.pts[0..k) (k >= 8) into
 // S.cand; S.fit_ok.  Every sum runs over the list in order, one thread each, with
 // the coordinates of kSeqAhead points loaded ahead of the dependent adds.
-__device__ void fit_list(const FundJob& J, FShared& S, double* jac, int k) {
+static __device__ void fit_list(const FundJob& J, FShared& S, double* jac, int k) {
   const int t = threadIdx.x;
   const double4* P = reinterpret_cast<const double4*>(J.pts);
   auto coord = [](const double4& p, int c) { return c == 0 ? p.x : c == 1 ? p.y : c == 2 ? p.z : p.w; };
@@ -804,7 +813,7 @@ __device__ void fit_list(const FundJob& J, FShared& S, double* jac, int k) {
 }
 
 // n == 7: fit_fundamental_7point and the best candidate (thread 0).
-__device__ void seven_point(const FundJob& J, FShared& S) {
+static __device__ void seven_point(const FundJob& J, FShared& S) {
   const int idx[7] = {0, 1, 2, 3, 4, 5, 6};
   M3 tq, tt;
   double ata[9][9];
@@ -850,7 +859,7 @@ __device__ void seven_point(const FundJob& J, FShared& S) {
     int cnt = 0;
     double err = 0.0;
     for (int i = 0; i < 7; ++i) {
-      const double d2 = sampson(f9, J.m[i]);
+      const double d2 = sampson(f9, J.xy[i]);
       if (d2 <= J.tsq) {
         ++cnt;
         err += d2;
@@ -867,12 +876,10 @@ __device__ void seven_point(const FundJob& J, FShared& S) {
   }
 }
 
-constexpr size_t kJacSmem = sizeof(double) * 162 * kFB;  // A and V of every sample of a batch
+static constexpr size_t kJacSmem = sizeof(double) * 162 * kFB;  // A and V of every sample of a batch
 
-__global__ void __launch_bounds__(kFThreads) fundamental_kernel(const FundJob* __restrict__ jobs) {
-  __shared__ FShared S;
+static __device__ void run(const FundJob& J, FShared& S) {
   extern __shared__ double jac[];
-  const FundJob& J = jobs[blockIdx.x];
   const int n = J.n, t = threadIdx.x;
   if (t == 0) {
     *J.has_f = 0;
@@ -880,7 +887,12 @@ __global__ void __launch_bounds__(kFThreads) fundamental_kernel(const FundJob* _
     if (J.iters) *J.iters = 0;
     S.have = 0;
   }
-  for (int i = t; i < n; i += kFThreads) J.mask[i] = 0;
+  for (int i = t; i < n; i += kFThreads) {
+    J.mask[i] = 0;
+    const psift_match& a = J.m[i];
+    J.xy[i] = make_float4(a.query_x, a.query_y, a.target_x, a.target_y);
+  }
+  __syncthreads();
   if (n < 7) return;
   if (n == 7) {
     if (t == 0) seven_point(J, S);
@@ -1012,30 +1024,42 @@ __global__ void __launch_bounds__(kFThreads) fundamental_kernel(const FundJob* _
       // 3. inlier counts: warp w takes hypotheses w, w + 8, ...
       {
         const int lane = t & 31, warp = t >> 5;
-        // two hypotheses per pass over the matches (one load, two independent evaluations)
-        for (int h = warp; h < nb; h += 2 * (kFThreads / 32)) {
-          const int h2 = h + kFThreads / 32;
-          const bool v1 = S.fok[h] != 0, v2 = h2 < nb && S.fok[h2] != 0;
-          int c1 = 0, c2 = 0;
-          if (v1 || v2) {
-            double f1[9], f2[9];
-            for (int i = 0; i < 9; ++i) {
-              f1[i] = S.F[h][i];
-              f2[i] = h2 < nb ? S.F[h2][i] : 0.0;
-            }
-            for (int i = lane; i < n; i += 32) {
-              const psift_match& a = J.m[i];
-              c1 += v1 && sampson_in(f1, a, J.tsq);
-              c2 += v2 && sampson_in(f2, a, J.tsq);
-            }
+        // kPass hypotheses per pass over the matches (one load and conversion,
+        // independent evaluations).  A pass ends early once none of its hypotheses
+        // can reach the incumbent's count any more: the replay only asks whether a
+        // count is at least that, and it never falls.
+        const int best = S.best_count;
+        for (int h0 = warp; h0 < nb; h0 += kPass * (kFThreads / 32)) {
+          double f[kPass][9];
+          bool v[kPass], any = false;
+          int c[kPass];
+#pragma unroll
+          for (int u = 0; u < kPass; ++u) {
+            const int h = h0 + u * (kFThreads / 32);
+            v[u] = h < nb && S.fok[h] != 0;
+            any |= v[u];
+            c[u] = 0;
+#pragma unroll
+            for (int i = 0; i < 9; ++i) f[u][i] = v[u] ? S.F[h][i] : 0.0;
           }
-          for (int o = 16; o >= 1; o >>= 1) {
-            c1 += __shfl_xor_sync(0xffffffffu, c1, o);
-            c2 += __shfl_xor_sync(0xffffffffu, c2, o);
+          for (int i0 = 0; any && i0 < n; i0 += 32 * kCheck) {
+            const int i1 = min(i0 + 32 * kCheck, n);
+            for (int i = i0 + lane; i < i1; i += 32) {
+              const float4 a = J.xy[i];
+              const double x1 = a.x, y1 = a.y, x2 = a.z, y2 = a.w;
+#pragma unroll
+              for (int u = 0; u < kPass; ++u) c[u] += sampson_in(f[u], x1, y1, x2, y2, J.tsq);
+            }
+            any = false;
+#pragma unroll
+            for (int u = 0; u < kPass; ++u)
+              any |= v[u] && (int)__reduce_add_sync(0xffffffffu, (unsigned)c[u]) + n - i1 >= best;
           }
-          if (lane == 0) {
-            S.cnt[h] = c1;
-            if (h2 < nb) S.cnt[h2] = c2;
+#pragma unroll
+          for (int u = 0; u < kPass; ++u) {
+            const int h = h0 + u * (kFThreads / 32);
+            const int sum = (int)__reduce_add_sync(0xffffffffu, (unsigned)c[u]);
+            if (lane == 0 && h < nb) S.cnt[h] = sum;
           }
         }
       }
@@ -1123,7 +1147,7 @@ __global__ void __launch_bounds__(kFThreads) fundamental_kernel(const FundJob* _
   if (!S.have) return;
   int c = 0;
   for (int i = t; i < n; i += kFThreads) {
-    const bool in = sampson(S.best, J.m[i]) <= J.tsq;
+    const bool in = sampson(S.best, J.xy[i]) <= J.tsq;
     J.mask[i] = in ? 1 : 0;
     c += in;
   }
@@ -1133,6 +1157,22 @@ __global__ void __launch_bounds__(kFThreads) fundamental_kernel(const FundJob* _
     *J.has_f = 1;
     for (int i = 0; i < 9; ++i) J.f9[i] = S.best[i];
   }
+}
+};
+
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) fundamental_kernel(const FundJob* __restrict__ jobs) {
+  __shared__ typename FundCta<THREADS>::FShared S;
+  FundCta<THREADS>::run(jobs[blockIdx.x], S);
+}
+
+template <int THREADS>
+cudaError_t launch_fundamental(const FundJob* jobs, int n, cudaStream_t st) {
+  constexpr size_t smem = FundCta<THREADS>::kJacSmem;
+  cudaError_t e = ensure_smem_attr((const void*)fundamental_kernel<THREADS>, smem);
+  if (e != cudaSuccess) return e;
+  fundamental_kernel<THREADS><<<n, THREADS, smem, st>>>(jobs);
+  return cudaGetLastError();
 }
 
 psift_status validate_fundamental_options(psift_ctx* ctx, const psift_fundamental_options* o) {
@@ -1145,7 +1185,7 @@ psift_status validate_fundamental_options(psift_ctx* ctx, const psift_fundamenta
 psift_status run_fundamental(psift_ctx* ctx, const psift_fundamental_job* jobs, int n,
                              const psift_fundamental_options& o) {
   size_t bytes = sizeof(FundJob) * (size_t)n + 4096;
-  for (int i = 0; i < n; ++i) bytes += 48 * (size_t)jobs[i].n + 3 * 256;
+  for (int i = 0; i < n; ++i) bytes += 64 * (size_t)jobs[i].n + 4 * 256;
   psift_status st = arena_reserve(ctx, bytes);
   if (st != PSIFT_OK) return st;
   FundJob* d_jobs = (FundJob*)arena_alloc(ctx, sizeof(FundJob) * n);
@@ -1165,20 +1205,19 @@ psift_status run_fundamental(psift_ctx* ctx, const psift_fundamental_job* jobs, 
     F.cdf = (double*)arena_alloc(ctx, 8 * (size_t)J.n + 8);
     F.terms = (double*)arena_alloc(ctx, 8 * (size_t)J.n + 8);
     F.pts = (double*)arena_alloc(ctx, 32 * (size_t)J.n + 32);
+    F.xy = (float4*)arena_alloc(ctx, sizeof(float4) * (size_t)J.n + 16);
     F.mask = J.inlier_mask;
     F.f9 = J.f9;
     F.has_f = J.has_f;
     F.count = (int*)J.inlier_count;
     F.iters = (int*)J.iterations;
-    if (!F.pts) return set_error(ctx, PSIFT_ERR_INTERNAL, "fundamental workspace carve overflow");
+    if (!F.xy) return set_error(ctx, PSIFT_ERR_INTERNAL, "fundamental workspace carve overflow");
   }
   PSIFT_CUDA_TRY(ctx, cudaMemcpyAsync(d_jobs, hj.data(), sizeof(FundJob) * n, cudaMemcpyHostToDevice, ctx->stream));
   StageScope sc(ctx, STAGE_RANSAC);
-  cudaError_t ea = ensure_smem_attr((const void*)fundamental_kernel, kJacSmem);
-  if (ea != cudaSuccess) return cuda_error(ctx, ea, "cudaFuncSetAttribute(fundamental_kernel)");
-  fundamental_kernel<<<n, kFThreads, kJacSmem, ctx->stream>>>(d_jobs);
+  const cudaError_t e = n <= ctx->num_sms ? launch_fundamental<512>(d_jobs, n, ctx->stream)
+                                          : launch_fundamental<256>(d_jobs, n, ctx->stream);
   ctx->launches++;
-  cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_error(ctx, e, "fundamental_ransac");
   return PSIFT_OK;
 }
