@@ -6,10 +6,10 @@
 // the forward pass rounds weights and activations to bf16 (round to nearest even)
 // and accumulates in f32.  The backward pass is f32 on the same bf16-rounded
 // operands (straight-through rounding).  Training is deterministic:
-//   mlp_fwd_bwd_kernel   one thread per sample: forward, dL/dz for every layer;
-//   mlp_grad_partial_kernel / mlp_grad_reduce_kernel: per-parameter sums over
-//                        chunks of samples in order, then over the chunks in order;
-//   mlp_adam_kernel      Adam update of the f32 masters.
+//   mlp_step_kernel    a CTA per chunk of samples: forward, dL/dz for every layer,
+//                      per-parameter sums over the chunk's samples in order;
+//   mlp_update_kernel  sums over the chunks in order, Adam update of the f32 masters,
+//                      the minibatch loss.
 // Loss: mean binary cross-entropy over the minibatch.
 #include <algorithm>
 
@@ -49,34 +49,26 @@ __device__ void load_params(const float* __restrict__ p, MlpSmem& s) {
   __syncthreads();
 }
 
-// Forward of one sample; returns z3 and fills xb, h1b (and z1 signs) on request.
-__device__ __forceinline__ float forward1(const MlpSmem& s, const float* __restrict__ x, float (&xb)[kF],
-                                          float (&h1b)[kH], float* h2b_out, uint64_t* z1pos, uint64_t* z2pos) {
+// Forward of one sample; returns z3.
+__device__ __forceinline__ float forward1(const MlpSmem& s, const float* __restrict__ x) {
+  float xb[kF], h1b[kH];
 #pragma unroll
   for (int k = 0; k < kF; ++k) xb[k] = bf16r(x[k]);
-  uint64_t p1 = 0;
 #pragma unroll
   for (int j = 0; j < kH; ++j) {
     float z = s.b1[j];
 #pragma unroll
     for (int k = 0; k < kF; ++k) z = __fmaf_rn(s.w1[j][k], xb[k], z);
-    p1 |= (z > 0.0f ? 1ull : 0ull) << j;
     h1b[j] = bf16r(z > 0.0f ? z : 0.0f);
   }
   float z3 = s.b3;
-  uint64_t p2 = 0;
 #pragma unroll 4
   for (int j = 0; j < kH; ++j) {
     float z = s.b2[j];
 #pragma unroll
     for (int k = 0; k < kH; ++k) z = __fmaf_rn(s.w2[j][k], h1b[k], z);
-    p2 |= (z > 0.0f ? 1ull : 0ull) << j;
-    const float h2 = bf16r(z > 0.0f ? z : 0.0f);
-    if (h2b_out) h2b_out[j] = h2;
-    z3 = __fmaf_rn(s.w3[j], h2, z3);
+    z3 = __fmaf_rn(s.w3[j], bf16r(z > 0.0f ? z : 0.0f), z3);
   }
-  if (z1pos) *z1pos = p1;
-  if (z2pos) *z2pos = p2;
   return z3;
 }
 
@@ -87,130 +79,253 @@ __global__ void __launch_bounds__(256) mlp_infer_kernel(const float* __restrict_
   __shared__ MlpSmem s;
   load_params(params, s);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    float xb[kF], h1b[kH];
-    const float z3 = forward1(s, X + (size_t)i * kF, xb, h1b, nullptr, nullptr, nullptr);
-    prob[i] = sigmoidf_(z3);
+    prob[i] = sigmoidf_(forward1(s, X + (size_t)i * kF));
   }
 }
 
-// One thread per minibatch sample b (sample index idx[b]).  Stores the operands
-// and deltas the per-parameter gradient sums need.
-__global__ void __launch_bounds__(128) mlp_fwd_bwd_kernel(const float* __restrict__ params,
-                                                          const float* __restrict__ X, const float* __restrict__ Y,
-                                                          const int* __restrict__ idx, int B, float* __restrict__ xb_o,
-                                                          float* __restrict__ h1b_o, float* __restrict__ h2b_o,
-                                                          float* __restrict__ dz1_o, float* __restrict__ dz2_o,
-                                                          float* __restrict__ dz3_o, float* __restrict__ loss_o) {
-  __shared__ MlpSmem s;
-  load_params(params, s);
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= B) return;
-  const int i = idx ? idx[b] : b;
-  float xb[kF], h1b[kH], h2b[kH];
-  uint64_t p1, p2;
-  const float z3 = forward1(s, X + (size_t)i * kF, xb, h1b, h2b, &p1, &p2);
-  const float p = sigmoidf_(z3);
-  const float y = Y[i];
-  // BCE with logits: softplus(z) - y z, numerically stable form
-  const float l = fmaxf(z3, 0.0f) - z3 * y + log1pf(expf(-fabsf(z3)));
-  const float invB = 1.0f / (float)B;
-  const float dz3 = (p - y) * invB;
-  float dz2[kH];
-#pragma unroll
-  for (int j = 0; j < kH; ++j) dz2[j] = ((p2 >> j) & 1ull) ? dz3 * s.w3[j] : 0.0f;
-#pragma unroll 4
-  for (int k = 0; k < kH; ++k) {
-    float dh = 0.0f;
-#pragma unroll
-    for (int j = 0; j < kH; ++j) dh = __fmaf_rn(s.w2[j][k], dz2[j], dh);
-    dz1_o[(size_t)b * kH + k] = ((p1 >> k) & 1ull) ? dh : 0.0f;
-  }
-#pragma unroll
-  for (int j = 0; j < kH; ++j) {
-    h1b_o[(size_t)b * kH + j] = h1b[j];
-    h2b_o[(size_t)b * kH + j] = h2b[j];
-    dz2_o[(size_t)b * kH + j] = dz2[j];
-  }
-#pragma unroll
-  for (int k = 0; k < kF; ++k) xb_o[(size_t)b * kF + k] = xb[k];
-  dz3_o[b] = dz3;
-  loss_o[b] = l;
-}
-
-// Gradient sums, deterministic: the batch is cut into chunks of kGradChunk
-// samples; mlp_grad_partial_kernel (one thread per (parameter, chunk)) sums a
-// chunk in sample order, mlp_grad_reduce_kernel adds the chunks' sums in chunk
-// order.  Fixed order, so every run gives the same bits.
+// One training step's samples, forward and backward, and their gradient sums: a CTA
+// per chunk of kGradChunk samples, everything in shared memory.  The three 128 x 64 x
+// 64 products (layer 2, its transpose, the W2 gradient) are register-tiled: a thread
+// holds 4 x 4 (or 4 x 2) results and takes one step of the inner index at a time, so
+// every result is the same chain of fused multiply-adds, in the same order, as one
+// thread per sample (or per parameter) would compute.  Deterministic: parameter sums
+// run over the chunk's samples in order, the chunks are added in order by
+// mlp_update_kernel.
+// Bound by shared-memory loads and the FP32 pipe (3 x 4096 cycles per chunk): a step
+// of 4096 samples takes 32 CTAs; as separate one-thread-per-sample and
+// one-thread-per-parameter kernels through global memory it was latency bound.
 constexpr int kGradChunk = 128;
+constexpr int kStepThreads = 512;
+constexpr int kSS = kGradChunk + 4;  // row stride of [unit][sample] arrays
+constexpr int kHS = kH + 4;          // row stride of [sample][unit] and weight arrays
+constexpr int kXS = kF + 4;          // row stride of the features
 
-__global__ void mlp_grad_partial_kernel(int B, const float* __restrict__ xb, const float* __restrict__ h1b,
-                                        const float* __restrict__ h2b, const float* __restrict__ dz1,
-                                        const float* __restrict__ dz2, const float* __restrict__ dz3,
-                                        float* __restrict__ partial) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= kNP) return;
-  const int b0 = blockIdx.y * kGradChunk;
-  const int b1 = min(B, b0 + kGradChunk);
-  float g = 0.0f;
-  if (p < kOffB1) {
-    const int j = (p - kOffW1) / kF, k = (p - kOffW1) % kF;
-    for (int b = b0; b < b1; ++b) g = __fmaf_rn(dz1[(size_t)b * kH + j], xb[(size_t)b * kF + k], g);
-  } else if (p < kOffW2) {
-    const int j = p - kOffB1;
-    for (int b = b0; b < b1; ++b) g += dz1[(size_t)b * kH + j];
-  } else if (p < kOffB2) {
-    const int j = (p - kOffW2) / kH, k = (p - kOffW2) % kH;
-    for (int b = b0; b < b1; ++b) g = __fmaf_rn(dz2[(size_t)b * kH + j], h1b[(size_t)b * kH + k], g);
-  } else if (p < kOffW3) {
-    const int j = p - kOffB2;
-    for (int b = b0; b < b1; ++b) g += dz2[(size_t)b * kH + j];
-  } else if (p < kOffB3) {
-    const int j = p - kOffW3;
-    for (int b = b0; b < b1; ++b) g = __fmaf_rn(dz3[b], h2b[(size_t)b * kH + j], g);
-  } else {
-    for (int b = b0; b < b1; ++b) g += dz3[b];
-  }
-  partial[(size_t)blockIdx.y * kNP + p] = g;
+struct StepSmem {
+  float w2[kH][kHS];    // [j][k]
+  float w2t[kH][kHS];   // [k][j]
+  float t[kH][kSS];     // h1 [k][sample], then dz2 [j][sample]
+  float h1[kGradChunk][kHS];  // activations: +0 where z <= 0, never elsewhere (see relu_bf16)
+  float h2[kGradChunk][kHS];
+  float dz2[kGradChunk][kHS];
+  float dz1[kGradChunk][kHS];
+  float x[kGradChunk][kXS];
+  float w1[kH][kF];
+  float b1[kH], b2[kH], w3[kH];
+  float dz3[kGradChunk];
+  float b3;
+};
+
+// bf16(max(z, 0)), with -0 for a positive z that rounds to zero: the bits are zero
+// exactly where the ReLU is inactive.
+__device__ __forceinline__ float relu_bf16(float z) {
+  if (!(z > 0.0f)) return 0.0f;
+  const float h = bf16r(z);
+  return h == 0.0f ? -0.0f : h;
 }
+__device__ __forceinline__ bool active(float h) { return __float_as_uint(h) != 0u; }
 
-__global__ void mlp_grad_reduce_kernel(int chunks, const float* __restrict__ partial, float* __restrict__ grad) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kStepThreads) mlp_step_kernel(const float* __restrict__ params,
+                                                                const float* __restrict__ X,
+                                                                const float* __restrict__ Y,
+                                                                const int* __restrict__ idx, int B,
+                                                                float* __restrict__ loss_o,
+                                                                float* __restrict__ partial) {
+  extern __shared__ __align__(16) uint8_t step_smem[];
+  StepSmem& s = *reinterpret_cast<StepSmem*>(step_smem);
+  const int tid = threadIdx.x;
+  const int b0 = blockIdx.x * kGradChunk, nb = min(kGradChunk, B - b0);
+  // parameters (weights rounded to bf16) and the chunk's features
+  for (int i = tid; i < kH * kF; i += kStepThreads) (&s.w1[0][0])[i] = bf16r(params[kOffW1 + i]);
+  for (int i = tid; i < kH * kH; i += kStepThreads) {
+    const float w = bf16r(params[kOffW2 + i]);
+    s.w2[i / kH][i % kH] = w;
+    s.w2t[i % kH][i / kH] = w;
+  }
+  if (tid < kH) {
+    s.b1[tid] = params[kOffB1 + tid];
+    s.b2[tid] = params[kOffB2 + tid];
+    s.w3[tid] = bf16r(params[kOffW3 + tid]);
+  }
+  if (tid == 0) s.b3 = params[kOffB3];
+  for (int i = tid; i < kGradChunk * kF; i += kStepThreads) {
+    const int r = i / kF, k = i % kF;
+    s.x[r][k] = r < nb ? bf16r(X[(size_t)(idx ? idx[b0 + r] : b0 + r) * kF + k]) : 0.0f;
+  }
+  __syncthreads();
+  // layer 1: a warp shares the unit j, lanes are samples
+  for (int i = tid; i < kGradChunk * kH; i += kStepThreads) {
+    const int r = i % kGradChunk, j = i / kGradChunk;
+    float z = s.b1[j];
+#pragma unroll
+    for (int k = 0; k < kF; ++k) z = __fmaf_rn(s.w1[j][k], s.x[r][k], z);
+    const float h = relu_bf16(z);
+    s.t[j][r] = h;
+    s.h1[r][j] = h;
+  }
+  __syncthreads();
+  // 4 x 4 tiles: a warp covers 32 samples x 16 units, lanes 8 x 4 tiles (two
+  // conflict-free 128-bit loads per step)
+  const int lane = tid & 31, warp = tid >> 5;
+  const int r0 = 32 * (warp & 3) + 4 * (lane & 7), u0 = 16 * (warp >> 2) + 4 * (lane >> 3);
+  {  // layer 2
+    float acc[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = s.b2[u0 + j];
+#pragma unroll 4
+    for (int k = 0; k < kH; ++k) {
+      const float4 h = *reinterpret_cast<const float4*>(&s.t[k][r0]), w = *reinterpret_cast<const float4*>(&s.w2t[k][u0]);
+      const float hv[4] = {h.x, h.y, h.z, h.w}, wv[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = __fmaf_rn(wv[j], hv[i], acc[i][j]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      *reinterpret_cast<float4*>(&s.h2[r0 + i][u0]) =
+          make_float4(relu_bf16(acc[i][0]), relu_bf16(acc[i][1]), relu_bf16(acc[i][2]), relu_bf16(acc[i][3]));
+    }
+  }
+  __syncthreads();
+  // layer 3, loss and its derivative: a thread per sample
+  if (tid < kGradChunk) {
+    float z3 = s.b3;
+#pragma unroll 4
+    for (int j = 0; j < kH; j += 4) {
+      const float4 h = *reinterpret_cast<const float4*>(&s.h2[tid][j]);
+      z3 = __fmaf_rn(s.w3[j], h.x, z3);
+      z3 = __fmaf_rn(s.w3[j + 1], h.y, z3);
+      z3 = __fmaf_rn(s.w3[j + 2], h.z, z3);
+      z3 = __fmaf_rn(s.w3[j + 3], h.w, z3);
+    }
+    float dz3 = 0.0f;
+    if (tid < nb) {
+      const float y = Y[idx ? idx[b0 + tid] : b0 + tid];
+      const float p = sigmoidf_(z3);
+      // BCE with logits: softplus(z) - y z, numerically stable form
+      loss_o[b0 + tid] = fmaxf(z3, 0.0f) - z3 * y + log1pf(expf(-fabsf(z3)));
+      dz3 = (p - y) * (1.0f / (float)B);
+    }
+    s.dz3[tid] = dz3;
+  }
+  __syncthreads();
+  for (int i = tid; i < kGradChunk * kH; i += kStepThreads) {
+    const int r = i % kGradChunk, j = i / kGradChunk;
+    const float d = active(s.h2[r][j]) ? s.dz3[r] * s.w3[j] : 0.0f;
+    s.t[j][r] = d;
+    s.dz2[r][j] = d;
+  }
+  __syncthreads();
+  {  // back through layer 2
+    float acc[4][4] = {};
+#pragma unroll 4
+    for (int j = 0; j < kH; ++j) {
+      const float4 d = *reinterpret_cast<const float4*>(&s.t[j][r0]), w = *reinterpret_cast<const float4*>(&s.w2[j][u0]);
+      const float dv[4] = {d.x, d.y, d.z, d.w}, wv[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) acc[i][k] = __fmaf_rn(wv[k], dv[i], acc[i][k]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) acc[i][k] = active(s.h1[r0 + i][u0 + k]) ? acc[i][k] : 0.0f;
+      *reinterpret_cast<float4*>(&s.dz1[r0 + i][u0]) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    }
+  }
+  __syncthreads();
+  float* part = partial + (size_t)blockIdx.x * kNP;
+  {  // W2 gradient: 4 (j) x 2 (k) per thread, lanes 4 x 8 tiles
+    const int j0 = 16 * (warp & 3) + 4 * (lane & 3), k0 = 16 * (warp >> 2) + 2 * (lane >> 2);
+    float acc[4][2] = {};
+#pragma unroll 4
+    for (int b = 0; b < nb; ++b) {
+      const float4 d = *reinterpret_cast<const float4*>(&s.dz2[b][j0]);
+      const float2 h = *reinterpret_cast<const float2*>(&s.h1[b][k0]);
+      const float dv[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        acc[j][0] = __fmaf_rn(dv[j], h.x, acc[j][0]);
+        acc[j][1] = __fmaf_rn(dv[j], h.y, acc[j][1]);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int k = 0; k < 2; ++k) part[kOffW2 + (j0 + j) * kH + k0 + k] = acc[j][k];
+  }
+  {  // W1 gradient: a parameter per thread
+    const int j = tid / kF, k = tid % kF;
+    float g = 0.0f;
+#pragma unroll 8
+    for (int b = 0; b < nb; ++b) g = __fmaf_rn(s.dz1[b][j], s.x[b][k], g);
+    part[kOffW1 + tid] = g;
+  }
+  // biases and W3
+  if (tid < 3 * kH + 1) {
+    const int j = tid % kH;
+    float g = 0.0f;
+    if (tid < kH) {
+#pragma unroll 8
+      for (int b = 0; b < nb; ++b) g += s.dz1[b][j];
+      part[kOffB1 + j] = g;
+    } else if (tid < 2 * kH) {
+#pragma unroll 8
+      for (int b = 0; b < nb; ++b) g += s.dz2[b][j];
+      part[kOffB2 + j] = g;
+    } else if (tid < 3 * kH) {
+#pragma unroll 8
+      for (int b = 0; b < nb; ++b) g = __fmaf_rn(s.dz3[b], s.h2[b][j], g);
+      part[kOffW3 + j] = g;
+    } else {
+#pragma unroll 8
+      for (int b = 0; b < nb; ++b) g += s.dz3[b];
+      part[kOffB3] = g;
+    }
+  }
+}
+static_assert(sizeof(StepSmem) <= 227 * 1024, "one chunk per SM");
+static_assert(kStepThreads == kH * kF && kGradChunk * kH == 16 * kStepThreads, "tiles cover the chunk");
+
+// Adds the chunks' gradient sums in chunk order and, with `update`, takes the Adam step
+// on the f32 masters; the last CTA writes the mean of the per-sample losses, in a fixed
+// order: thread t sums samples t, t + 256, t + 512, ..., then a fixed pairwise tree.
+constexpr int kUpdateThreads = 256;
+__global__ void __launch_bounds__(kUpdateThreads) mlp_update_kernel(
+    int chunks, const float* __restrict__ partial, float* __restrict__ grad, float* __restrict__ params,
+    float* __restrict__ m, float* __restrict__ v, bool update, float lr, float beta1, float beta2, float eps, float bc1,
+    float bc2, const float* __restrict__ l, int B, float* __restrict__ loss_out) {
+  __shared__ float part[kUpdateThreads];
+  const int t = threadIdx.x;
+  if (blockIdx.x == gridDim.x - 1) {
+    if (!loss_out) return;
+    float sum = 0.0f;
+    for (int b = t; b < B; b += kUpdateThreads) sum += l[b];
+    part[t] = sum;
+    __syncthreads();
+    for (int h = kUpdateThreads / 2; h > 0; h >>= 1) {
+      if (t < h) part[t] += part[t + h];
+      __syncthreads();
+    }
+    if (t == 0) *loss_out = part[0] / (float)B;
+    return;
+  }
+  const int p = blockIdx.x * kUpdateThreads + t;
   if (p >= kNP) return;
   float g = 0.0f;
+#pragma unroll 8
   for (int c = 0; c < chunks; ++c) g += partial[(size_t)c * kNP + p];
   grad[p] = g;
-}
-
-__global__ void mlp_adam_kernel(float* __restrict__ params, const float* __restrict__ grad, float* __restrict__ m,
-                                float* __restrict__ v, float lr, float beta1, float beta2, float eps, float bc1,
-                                float bc2) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= kNP) return;
-  const float g = grad[p];
-  const float mm = beta1 * m[p] + (1.0f - beta1) * g;
-  const float vv = beta2 * v[p] + (1.0f - beta2) * g * g;
-  m[p] = mm;
-  v[p] = vv;
-  params[p] -= lr * (mm / bc1) / (sqrtf(vv / bc2) + eps);
-}
-
-// Mean of the per-sample losses into loss[step], in a fixed order (deterministic):
-// thread t sums samples t, t + 256, t + 512, ... in that order (coalesced loads
-// across a warp), then a fixed pairwise tree over the 256 partial sums.  One CTA.
-constexpr int kLossThreads = 256;
-__global__ void __launch_bounds__(kLossThreads) mlp_loss_kernel(const float* __restrict__ l, int B,
-                                                                float* __restrict__ out) {
-  __shared__ float part[kLossThreads];
-  const int t = threadIdx.x;
-  float s = 0.0f;
-  for (int b = t; b < B; b += kLossThreads) s += l[b];
-  part[t] = s;
-  __syncthreads();
-  for (int h = kLossThreads / 2; h > 0; h >>= 1) {
-    if (t < h) part[t] += part[t + h];
-    __syncthreads();
+  if (update) {
+    const float mm = beta1 * m[p] + (1.0f - beta1) * g;
+    const float vv = beta2 * v[p] + (1.0f - beta2) * g * g;
+    m[p] = mm;
+    v[p] = vv;
+    params[p] -= lr * (mm / bc1) / (sqrtf(vv / bc2) + eps);
   }
-  if (t == 0) *out = part[0] / (float)B;
 }
 
 // ------------------------------------------------------------ tensor-core inference
@@ -414,33 +529,23 @@ cudaError_t launch_mlp_infer(const float* params, const float* X, int n, float* 
   return cudaGetLastError();
 }
 
-// Workspace for a minibatch of B: (8 + 64*4 + 2) * B floats of per-sample
-// operands, then one row of kNP partial gradient sums per kGradChunk samples.
-size_t mlp_batch_floats(int B) {
-  return (size_t)B * (kF + 4 * kH + 2) + (size_t)((B + kGradChunk - 1) / kGradChunk) * kNP;
-}
+// Workspace for a minibatch of B: the per-sample losses, then one row of kNP partial
+// gradient sums per kGradChunk samples.
+size_t mlp_batch_floats(int B) { return (size_t)B + (size_t)((B + kGradChunk - 1) / kGradChunk) * kNP; }
 
 cudaError_t launch_mlp_step(float* params, const float* X, const float* Y, const int* idx, int B, float* work,
                             float* grad, float* m, float* v, float lr, int t, float* loss_out, bool update,
                             cudaStream_t st) {
-  float* xb = work;
-  float* h1b = xb + (size_t)B * kF;
-  float* h2b = h1b + (size_t)B * kH;
-  float* dz1 = h2b + (size_t)B * kH;
-  float* dz2 = dz1 + (size_t)B * kH;
-  float* dz3 = dz2 + (size_t)B * kH;
-  float* lb = dz3 + B;
+  float* lb = work;
   float* partial = lb + B;
   const int chunks = (B + kGradChunk - 1) / kGradChunk;
-  mlp_fwd_bwd_kernel<<<(B + 127) / 128, 128, 0, st>>>(params, X, Y, idx, B, xb, h1b, h2b, dz1, dz2, dz3, lb);
-  mlp_grad_partial_kernel<<<dim3((kNP + 127) / 128, chunks), 128, 0, st>>>(B, xb, h1b, h2b, dz1, dz2, dz3, partial);
-  mlp_grad_reduce_kernel<<<(kNP + 127) / 128, 128, 0, st>>>(chunks, partial, grad);
-  if (loss_out) mlp_loss_kernel<<<1, kLossThreads, 0, st>>>(lb, B, loss_out);
-  if (update) {
-    const float b1 = 0.9f, b2 = 0.999f;
-    const float bc1 = 1.0f - powf(b1, (float)t), bc2 = 1.0f - powf(b2, (float)t);
-    mlp_adam_kernel<<<(kNP + 255) / 256, 256, 0, st>>>(params, grad, m, v, lr, b1, b2, 1e-8f, bc1, bc2);
-  }
+  cudaError_t e = ensure_smem_attr((const void*)mlp_step_kernel, sizeof(StepSmem));
+  if (e != cudaSuccess) return e;
+  mlp_step_kernel<<<chunks, kStepThreads, sizeof(StepSmem), st>>>(params, X, Y, idx, B, lb, partial);
+  const float b1 = 0.9f, b2 = 0.999f;
+  const float bc1 = 1.0f - powf(b1, (float)t), bc2 = 1.0f - powf(b2, (float)t);
+  mlp_update_kernel<<<(kNP + kUpdateThreads - 1) / kUpdateThreads + 1, kUpdateThreads, 0, st>>>(
+      chunks, partial, grad, params, m, v, update, lr, b1, b2, 1e-8f, bc1, bc2, lb, B, loss_out);
   return cudaGetLastError();
 }
 
