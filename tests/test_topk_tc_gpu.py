@@ -1,0 +1,55 @@
+"""The tensor-core Hamming shortlist: lists equal to the CPU restatement's where ranges,
+tiles and blocks end, with crowded distances, and where the candidates overflow."""
+import numpy as np
+import pytest
+
+import oracle as O
+import psift
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(q, c, k, ctx=None):
+    gi, gd = psift.hamming_topk(q, c, k, ctx=ctx)
+    ri, rd = O.hamming_topk(q, c, k)
+    np.testing.assert_array_equal(gd, rd)
+    np.testing.assert_array_equal(gi, ri)
+
+
+# 65536 codes and 64 queries are the smallest it takes; 512-code blocks, 256-code tiles,
+# 128-query tiles, ranges of 8x from max(n / 64, 4096)
+@pytest.mark.parametrize("nq,ncat,k", [(64, 65536, 64), (65, 65537, 1), (128, 66047, 64), (129, 66048, 33),
+                                       (300, 262657, 64), (1000, 300000, 16)])
+def test_lists_equal_the_oracle(nq, ncat, k):
+    rng = np.random.default_rng(nq + ncat)
+    c = rng.integers(0, 2 ** 64, (ncat, 2), dtype=np.uint64)
+    q = rng.integers(0, 2 ** 64, (nq, 2), dtype=np.uint64)
+    q[: nq // 2] = c[rng.integers(0, ncat, nq // 2)] ^ np.uint64(5)
+    _check(q, c, k)
+
+
+def test_crowded_distances():
+    # few distinct codes: most distances tie, the index decides
+    rng = np.random.default_rng(3)
+    pool = rng.integers(0, 2 ** 64, (7, 2), dtype=np.uint64)
+    c = pool[rng.integers(0, 7, 70001)]
+    q = np.concatenate([pool[rng.integers(0, 7, 60)], rng.integers(0, 2 ** 64, (40, 2), dtype=np.uint64)])
+    _check(q, c, 64)
+    _check(q, np.zeros_like(c), 64)
+    _check(np.zeros_like(q), ~np.zeros_like(c), 64)
+
+
+def test_candidates_that_overflow():
+    # every code of the last third is nearer to the first queries than all before it
+    rng = np.random.default_rng(4)
+    c = rng.integers(0, 2 ** 64, (90000, 2), dtype=np.uint64)
+    q = rng.integers(0, 2 ** 64, (80, 2), dtype=np.uint64)
+    noise = np.uint64(1) << rng.integers(0, 64, 30000, dtype=np.uint64)
+    c[60000:, 0] = q[0, 0] ^ noise
+    c[60000:, 1] = q[0, 1]
+    q[1] = q[0]
+    q[2] = ~q[0]
+    ctx = psift.Context(0)
+    for k in (1, 40, 64):
+        _check(q, c, k, ctx)
+    ctx.close()
