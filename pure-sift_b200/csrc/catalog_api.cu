@@ -15,15 +15,10 @@ cudaError_t launch_popc_probe(int blocks, int iters, uint32_t* out, cudaStream_t
 cudaError_t launch_dequantize(const uint8_t* q, int n, float* out, cudaStream_t st);
 cudaError_t launch_votes(const uint64_t* q, int nq, const uint64_t* cat, const long long* offsets, int n_entries,
                          int mih, uint32_t* votes, cudaStream_t st);
-int topk_chunks(long long ncat, int nq, int num_sms);
-cudaError_t launch_topk(const uint64_t* q, int nq, const uint64_t* cat, long long ncat, int k, int n_chunks,
-                        unsigned long long* part, uint32_t* out_idx, uint32_t* out_dist, cudaStream_t st);
-bool topk_tc_applies(int nq, long long ncat);
-long long topk_tc_first(long long ncat);
-size_t topk_tc_scratch(int nq);
-cudaError_t launch_topk_tc(const uint64_t* q, int nq, const uint64_t* cat, long long ncat, int k, int first_chunks,
-                           unsigned long long* part, uint8_t* scratch, uint32_t* out_idx, uint32_t* out_dist,
-                           int num_sms, uint32_t* err, uint64_t* launches, cudaStream_t st);
+size_t topk_scratch(int nq, int block);
+cudaError_t launch_topk(const uint64_t* q, int nq, const uint64_t* cat, long long ncat, int k, int block,
+                        uint8_t* scratch, uint32_t* out_idx, uint32_t* out_dist, int num_sms, uint32_t* err,
+                        uint64_t* launches, cudaStream_t st);
 cudaError_t launch_l2_rerank(const float* qd, int nq, const float* cd, const uint32_t* cand, int k,
                              uint32_t* out_idx, float* out_d2, cudaStream_t st);
 
@@ -189,27 +184,14 @@ psift_status psift_hamming_topk_dev(psift_ctx* ctx, const uint64_t* q_codes, uin
   if (nq == 0) return PSIFT_OK;
   if (!q_codes || !idx || !dist || (ncat && !cat_codes)) return set_error(ctx, PSIFT_ERR_INVALID_ARGUMENT, "null argument");
   if (ncat >= 0xFFFFFFFFull) return set_error(ctx, PSIFT_ERR_INVALID_ARGUMENT, "catalog larger than 2^32-1 codes");
-  if (topk_tc_applies((int)nq, (long long)ncat)) {
-    const int first_chunks = topk_chunks(topk_tc_first((long long)ncat), (int)nq, ctx->num_sms);
-    const size_t part_bytes = (size_t)nq * first_chunks * k * 8;
-    if (arena_reserve(ctx, part_bytes + topk_tc_scratch((int)nq) + 4096) == PSIFT_OK) {
-      unsigned long long* part = (unsigned long long*)arena_alloc(ctx, part_bytes);
-      uint8_t* scratch = (uint8_t*)arena_alloc(ctx, topk_tc_scratch((int)nq));
-      StageScope sc(ctx, STAGE_HAMMING);
-      const cudaError_t e = launch_topk_tc(q_codes, (int)nq, cat_codes, (long long)ncat, (int)k, first_chunks, part,
-                                           scratch, idx, dist, ctx->num_sms, ctx->d_error, &ctx->launches, ctx->stream);
-      if (e != cudaSuccess) return cuda_error(ctx, e, "hamming_topk");
-      return PSIFT_OK;
-    }
-    // no room for its candidates: the popcount scan needs less
-  }
-  const int chunks = topk_chunks((long long)ncat, (int)nq, ctx->num_sms);
-  st = arena_reserve(ctx, (size_t)nq * chunks * k * 8 + 4096);
+  // 8192 queries at a time (8 KB of candidates each); fewer when the device is that full
+  int block = 8192;
+  while ((st = arena_reserve(ctx, topk_scratch((int)nq, block) + 4096)) != PSIFT_OK && block > 128) block /= 8;
   if (st != PSIFT_OK) return st;
-  unsigned long long* part = (unsigned long long*)arena_alloc(ctx, (size_t)nq * chunks * k * 8);
+  uint8_t* scratch = (uint8_t*)arena_alloc(ctx, topk_scratch((int)nq, block));
   StageScope sc(ctx, STAGE_HAMMING);
-  cudaError_t e = launch_topk(q_codes, (int)nq, cat_codes, (long long)ncat, (int)k, chunks, part, idx, dist, ctx->stream);
-  ctx->launches += 2;
+  const cudaError_t e = launch_topk(q_codes, (int)nq, cat_codes, (long long)ncat, (int)k, block, scratch, idx, dist,
+                                    ctx->num_sms, ctx->d_error, &ctx->launches, ctx->stream);
   if (e != cudaSuccess) return cuda_error(ctx, e, "hamming_topk");
   return PSIFT_OK;
 }

@@ -17,20 +17,15 @@
 // without the inverted tables.
 //
 // Top-k shortlist (no reference counterpart; the catalog search at scale): the k
-// codes nearest to each query by (Hamming distance, catalog index).  One warp
-// serves 16 queries over one chunk of codes: lane i scores code base+i against the
-// 16 queries (4 XOR + 4 POPC each); a ballot finds codes beating a query's current
-// k-th entry, and the warp replaces that entry cooperatively (rare after the list
-// fills).  Chunk lists are merged per query by a second kernel.
+// codes nearest to each query by (Hamming distance, catalog index), in hamming_tc.cu;
+// the exact f32 re-rank of a shortlist is here.
 #include <algorithm>
 
 #include "psift_internal.cuh"
 
 namespace psift {
 
-constexpr int kQG = 16;       // queries per warp
 constexpr int kTopKMax = 64;  // shortlist length upper bound
-constexpr int kHamWarps = 4;
 
 // popc(x0) + popc(x1) + popc(x2) + popc(x3) with three popcounts: a carry-save
 // step gives, bit by bit, x0 + x1 + x2 = s + 2c (s = x0 ^ x1 ^ x2, c = majority),
@@ -205,265 +200,6 @@ __global__ void __launch_bounds__(256) votes_kernel(const uint4* __restrict__ q,
   }
 }
 
-// Per (16-query group, code chunk): the k smallest (distance, index) keys.
-// Grid (n_chunks, ceil(n_groups / kHamWarps)), kHamWarps warps per block.
-//
-// Each query keeps its list sorted, entries [k, 64) at ~0, and maxd = the
-// distance of its k-th key.  Within a chunk the codes come in increasing index,
-// so every listed entry has a smaller index than the current code: a code can
-// only enter when its distance is below maxd.  Such codes are appended to the
-// query's buffer (up to kTopKBuf keys); a full buffer (and the buffer at the end
-// of the chunk) is merged into the list: the buffer sorted across the warp's
-// lanes, each key's place in the merged order found by binary search in the
-// other sorted sequence (ties: the list's key first; only the empty ~0 keys tie),
-// the first k kept.  A candidate that passed against an older maxd and no longer
-// belongs falls out at its merge.
-constexpr int kTopKBuf = 32;
-constexpr size_t kTopKWarpSmem = (size_t)kQG * (kTopKMax + kTopKBuf) * 8 + kTopKMax * 8 + kQG * 4;
-
-__device__ __forceinline__ unsigned long long shfl_xor_u64(unsigned long long v, int o) {
-  return __shfl_xor_sync(0xffffffffu, v, o);
-}
-
-// Merges buf[0..n) into the sorted list (k entries kept); returns the new k-th distance.
-__device__ __forceinline__ uint32_t topk_merge_buffer(unsigned long long* list, unsigned long long* buf, int n,
-                                                      int k, unsigned long long* scratch, int lane) {
-  __syncwarp();
-  // sort the buffer across the lanes (ascending; missing entries ~0)
-  unsigned long long v = lane < n ? buf[lane] : ~0ull;
-#pragma unroll
-  for (int kk = 2; kk <= 32; kk <<= 1) {
-#pragma unroll
-    for (int j = kk >> 1; j > 0; j >>= 1) {
-      const unsigned long long o = shfl_xor_u64(v, j);
-      const bool up = (lane & kk) == 0, low = (lane & j) == 0;
-      v = (low == up) ? (o < v ? o : v) : (o > v ? o : v);
-    }
-  }
-  buf[lane] = v;
-  __syncwarp();
-  // buffer key at lane: rank = lane + (list keys <= it)
-  {
-    int lo = 0, hi = kTopKMax;  // first list index with key > v
-    while (lo < hi) {
-      const int mid = (lo + hi) >> 1;
-      if (list[mid] <= v) lo = mid + 1;
-      else hi = mid;
-    }
-    const int r = lane + lo;
-    if (r < k) scratch[r] = v;
-  }
-  // list keys at lane and lane + 32: rank = i + (buffer keys < it)
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int i = lane + 32 * h;
-    const unsigned long long x = list[i];
-    int lo = 0, hi = 32;  // first buffer index with key >= x
-    while (lo < hi) {
-      const int mid = (lo + hi) >> 1;
-      if (buf[mid] < x) lo = mid + 1;
-      else hi = mid;
-    }
-    const int r = i + lo;
-    if (r < k) scratch[r] = x;
-  }
-  __syncwarp();
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int i = lane + 32 * h;
-    if (i < k) list[i] = scratch[i];
-  }
-  __syncwarp();
-  return (uint32_t)(list[k - 1] >> 32);
-}
-
-__global__ void __launch_bounds__(kHamWarps * 32, 4) topk_chunk_kernel(const uint4* __restrict__ q, int nq,
-                                                                        const uint4* __restrict__ cat, long long ncat,
-                                                                        int k, int n_chunks,
-                                                                        unsigned long long* __restrict__ part) {
-  extern __shared__ __align__(16) unsigned long long s_topk[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int group = blockIdx.y * kHamWarps + warp;
-  const int q0 = group * kQG;
-  if (q0 >= nq) return;
-  const int chunk = blockIdx.x;
-  const long long c_begin = ncat * chunk / n_chunks, c_end = ncat * (chunk + 1) / n_chunks;
-  unsigned long long* wbase = s_topk + (size_t)warp * (kTopKWarpSmem / 8);
-  unsigned long long(*list)[kTopKMax] = reinterpret_cast<unsigned long long(*)[kTopKMax]>(wbase);
-  unsigned long long(*buf)[kTopKBuf] = reinterpret_cast<unsigned long long(*)[kTopKBuf]>(wbase + kQG * kTopKMax);
-  unsigned long long* scratch = wbase + kQG * (kTopKMax + kTopKBuf);
-  uint32_t* cnt = reinterpret_cast<uint32_t*>(scratch + kTopKMax);
-  uint32_t qw[kQG][4];
-#pragma unroll
-  for (int j = 0; j < kQG; ++j) {
-    const uint4 v = (q0 + j < nq) ? q[q0 + j] : make_uint4(0, 0, 0, 0);
-    qw[j][0] = v.x;
-    qw[j][1] = v.y;
-    qw[j][2] = v.z;
-    qw[j][3] = v.w;
-  }
-  uint32_t maxd[kQG];
-#pragma unroll
-  for (int j = 0; j < kQG; ++j) {
-    list[j][lane] = ~0ull;
-    list[j][lane + 32] = ~0ull;
-    maxd[j] = 0xFFFFFFFFu;
-  }
-  if (lane < kQG) cnt[lane] = 0;
-  __syncwarp();
-  const unsigned lt = (1u << lane) - 1u;
-  // the next 32 codes are loaded while the current ones are compared
-  uint4 c_next = c_begin + lane < c_end ? cat[c_begin + lane] : make_uint4(0, 0, 0, 0);
-  for (long long base = c_begin; base < c_end; base += 32) {
-    const long long idx = base + lane;
-    const bool valid = idx < c_end;
-    const uint4 c = c_next;
-    c_next = idx + 32 < c_end ? cat[idx + 32] : make_uint4(0, 0, 0, 0);
-#pragma unroll
-    for (int j = 0; j < kQG; ++j) {
-      const uint32_t d = (uint32_t)ham128(qw[j][0], qw[j][1], qw[j][2], qw[j][3], c);
-      const unsigned m = __ballot_sync(0xffffffffu, valid && d < maxd[j]);
-      if (m) {
-        const int nc = __popc(m);
-        int n = (int)cnt[j];
-        if (n + nc > kTopKBuf) {
-          maxd[j] = topk_merge_buffer(list[j], buf[j], n, k, scratch, lane);
-          n = 0;
-        }
-        if (m & (1u << lane))
-          buf[j][n + __popc(m & lt)] = ((unsigned long long)d << 32) | (unsigned long long)(uint32_t)idx;
-        __syncwarp();
-        if (lane == 0) cnt[j] = (uint32_t)(n + nc);
-        __syncwarp();
-      }
-    }
-  }
-  // the buffers' last keys, then this chunk's lists: part[(query * n_chunks + chunk) * k + t]
-#pragma unroll
-  for (int j = 0; j < kQG; ++j) {
-    if (cnt[j] > 0) topk_merge_buffer(list[j], buf[j], (int)cnt[j], k, scratch, lane);
-    if (q0 + j >= nq) continue;
-    unsigned long long* dst = part + ((long long)(q0 + j) * n_chunks + chunk) * k;
-    for (int t = lane; t < k; t += 32) dst[t] = list[j][t];
-  }
-}
-
-// Ascending bitonic sort of a[0..m) (m a power of two) by one warp.
-__device__ __forceinline__ void warp_bitonic_u64(unsigned long long* a, int m, int lane) {
-  for (int kk = 2; kk <= m; kk <<= 1) {
-    for (int j = kk >> 1; j > 0; j >>= 1) {
-      for (int i = lane; i < m; i += 32) {
-        const int ixj = i ^ j;
-        if (ixj > i) {
-          const unsigned long long x = a[i], y = a[ixj];
-          const bool up = (i & kk) == 0;
-          if ((x > y) == up) {
-            a[i] = y;
-            a[ixj] = x;
-          }
-        }
-      }
-      __syncwarp();
-    }
-  }
-}
-
-// Per query (one warp): the k smallest of the chunks' n_chunks * k keys
-// (distance << 32 | index; empty slots ~0), ascending.  Keys are unique apart
-// from the empty slots (the chunks partition the catalog).  A histogram of the
-// distances (0..128, bin 129 for empty slots) gives the distance D of the k-th
-// smallest key and the count `below` of keys under D (< k).  Those keys are
-// compacted into `low`, the keys at D into the front of `keys` (in place: a
-// round writes only at or below the positions it has read), each group is
-// sorted, and the result is low[0..below) followed by the first k - below keys
-// at D, i.e. by index.  Shared memory per warp: keys[n2], low[64], hist[132].
-constexpr int kMergeBins = 130;
-constexpr int kMergeHist = 132;
-__global__ void topk_merge_kernel(const unsigned long long* __restrict__ part, int nq, int k, int n_chunks, int n2,
-                                  uint32_t* __restrict__ out_idx, uint32_t* __restrict__ out_dist) {
-  extern __shared__ unsigned long long s_keys[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int qi = blockIdx.x * (blockDim.x >> 5) + warp;
-  unsigned long long* keys = s_keys + (size_t)warp * (n2 + kTopKMax + kMergeHist / 2);
-  unsigned long long* low = keys + n2;
-  uint32_t* hist = reinterpret_cast<uint32_t*>(low + kTopKMax);
-  if (qi >= nq) return;
-  const int total = n_chunks * k;
-  const unsigned long long* src = part + (long long)qi * total;
-  for (int t = lane; t < kMergeHist; t += 32) hist[t] = 0;
-  for (int t = lane; t < total; t += 32) keys[t] = src[t];
-  __syncwarp();
-  auto bin_of = [](unsigned long long key) {
-    const uint32_t d = (uint32_t)(key >> 32);
-    return d <= 128u ? (int)d : kMergeBins - 1;
-  };
-  for (int t = lane; t < total; t += 32) atomicAdd(&hist[bin_of(keys[t])], 1u);
-  __syncwarp();
-  // D: the bin where the running count reaches k (lane l scans bins 5l .. 5l + 4)
-  int local = 0;
-#pragma unroll
-  for (int b = 0; b < 5; ++b) local += 5 * lane + b < kMergeBins ? (int)hist[5 * lane + b] : 0;
-  int incl = local;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int v = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += v;
-  }
-  const int excl = incl - local;
-  int my_d = -1, my_below = 0;
-  if (excl < k && incl >= k) {
-    int run = excl;
-    for (int b = 5 * lane; b < 5 * lane + 5; ++b) {
-      const int c = (int)hist[b];
-      if (run + c >= k) {
-        my_d = b;
-        my_below = run;
-        break;
-      }
-      run += c;
-    }
-  }
-  const int owner = __ffs(__ballot_sync(0xffffffffu, my_d >= 0)) - 1;
-  const int D = __shfl_sync(0xffffffffu, my_d, owner);
-  const int below = __shfl_sync(0xffffffffu, my_below, owner);
-  const int n_tie = (int)hist[D];
-  // compaction, in key order of the chunks
-  int n_low = 0, n_at = 0;
-  const unsigned lt = (1u << lane) - 1u;
-  for (int base = 0; base < total; base += 32) {
-    const int t = base + lane;
-    const unsigned long long key = t < total ? keys[t] : ~0ull;
-    const int b = t < total ? bin_of(key) : kMergeBins;
-    const unsigned ml = __ballot_sync(0xffffffffu, b < D);
-    const unsigned mt = __ballot_sync(0xffffffffu, b == D);
-    __syncwarp();
-    if (b < D) low[n_low + __popc(ml & lt)] = key;
-    if (b == D) keys[n_at + __popc(mt & lt)] = key;
-    n_low += __popc(ml);
-    n_at += __popc(mt);
-    __syncwarp();
-  }
-  // sort the group under D (padded to a power of two) and, unless they are all
-  // empty slots, the keys at D
-  int m = 1;
-  while (m < below) m <<= 1;
-  for (int t = below + lane; t < m; t += 32) low[t] = ~0ull;
-  int m2 = 1;
-  while (m2 < n_tie) m2 <<= 1;
-  const bool sort_tie = D < kMergeBins - 1 && n_tie > 1;
-  if (sort_tie)
-    for (int t = n_tie + lane; t < m2; t += 32) keys[t] = ~0ull;
-  __syncwarp();
-  if (below > 1) warp_bitonic_u64(low, m, lane);
-  if (sort_tie) warp_bitonic_u64(keys, m2, lane);
-  for (int t = lane; t < k; t += 32) {
-    const unsigned long long key = t < below ? low[t] : keys[t - below];
-    const bool ok = key != ~0ull;
-    out_idx[(long long)qi * k + t] = ok ? (uint32_t)(key & 0xFFFFFFFFu) : 0xFFFFFFFFu;
-    out_dist[(long long)qi * k + t] = ok ? (uint32_t)(key >> 32) : 0xFFFFFFFFu;
-  }
-}
-
 // Exact FP32 L2^2 re-rank of each query's k candidates (reference summation
 // order), sorted by (d2, index).  One warp per query.
 __global__ void l2_rerank_kernel(const float* __restrict__ qd, int nq, const float* __restrict__ cd,
@@ -482,9 +218,10 @@ __global__ void l2_rerank_kernel(const float* __restrict__ qd, int nq, const flo
       if (c != 0xFFFFFFFFu) {
         const float* b = cd + (size_t)c * 128;
         float s = 0.0f;
+#pragma unroll 8  // 8 of the row's loads in flight: a lane walks its own row, latency bound
         for (int i = 0; i < 128; i += 4) {
-          const float4 x = *reinterpret_cast<const float4*>(a + i);
-          const float4 y = *reinterpret_cast<const float4*>(b + i);
+          const float4 x = __ldg(reinterpret_cast<const float4*>(a + i));
+          const float4 y = __ldg(reinterpret_cast<const float4*>(b + i));
           float d = x.x - y.x;
           s += d * d;
           d = x.y - y.y;
@@ -542,37 +279,6 @@ cudaError_t launch_votes(const uint64_t* q, int nq, const uint64_t* cat, const l
                          int mih, uint32_t* votes, cudaStream_t st) {
   if (n_entries <= 0) return cudaSuccess;
   votes_kernel<<<n_entries, 256, 0, st>>>((const uint4*)q, nq, (const uint4*)cat, offsets, mih, votes);
-  return cudaGetLastError();
-}
-
-int topk_chunks(long long ncat, int nq, int num_sms) {
-  const int groups = (nq + kQG - 1) / kQG;
-  long long want = (long long)num_sms * 16 * 2 / std::max(groups, 1);  // ~2 waves of 16 warps per SM
-  want = std::max<long long>(1, std::min<long long>(want, 64));
-  want = std::min<long long>(want, std::max<long long>(1, ncat / 1024));
-  return (int)want;
-}
-
-cudaError_t launch_topk(const uint64_t* q, int nq, const uint64_t* cat, long long ncat, int k, int n_chunks,
-                        unsigned long long* part, uint32_t* out_idx, uint32_t* out_dist, cudaStream_t st) {
-  if (nq <= 0) return cudaSuccess;
-  const int groups = (nq + kQG - 1) / kQG;
-  dim3 g1(n_chunks, (groups + kHamWarps - 1) / kHamWarps);
-  const size_t smem1 = kHamWarps * kTopKWarpSmem;
-  cudaError_t e = ensure_smem_attr((const void*)topk_chunk_kernel, smem1);
-  if (e != cudaSuccess) return e;
-  topk_chunk_kernel<<<g1, kHamWarps * 32, smem1, st>>>((const uint4*)q, nq, (const uint4*)cat, ncat, k, n_chunks,
-                                                      part);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  int n2 = 1;
-  while (n2 < n_chunks * k) n2 <<= 1;
-  const size_t per_warp = ((size_t)n2 + kTopKMax + kMergeHist / 2) * 8;
-  const int warps = std::max(1, std::min(8, (int)(96 * 1024 / per_warp)));
-  const size_t smem = (size_t)warps * per_warp;
-  e = ensure_smem_attr((const void*)topk_merge_kernel, smem);
-  if (e != cudaSuccess) return e;
-  topk_merge_kernel<<<(nq + warps - 1) / warps, warps * 32, smem, st>>>(part, nq, k, n_chunks, n2, out_idx, out_dist);
   return cudaGetLastError();
 }
 

@@ -16,16 +16,24 @@ def _check(q, c, k, ctx=None):
     np.testing.assert_array_equal(gi, ri)
 
 
-# 65536 codes and 64 queries are the smallest it takes; 512-code blocks, 256-code tiles,
-# 128-query tiles, ranges of 8x from max(n / 64, 4096)
-@pytest.mark.parametrize("nq,ncat,k", [(64, 65536, 64), (65, 65537, 1), (128, 66047, 64), (129, 66048, 33),
-                                       (300, 262657, 64), (1000, 300000, 16)])
+# the first 2048 codes are listed directly; then 512-code blocks, 256-code tiles, 128-query
+# tiles, ranges of 8x
+@pytest.mark.parametrize("nq,ncat,k", [(1, 1, 1), (3, 40, 64), (5, 2047, 64), (5, 2048, 64), (1, 2049, 64),
+                                       (127, 2305, 7), (128, 2561, 64), (129, 16384, 33), (65, 16385, 1),
+                                       (300, 131073, 64), (64, 262657, 64), (1000, 300000, 16)])
 def test_lists_equal_the_oracle(nq, ncat, k):
     rng = np.random.default_rng(nq + ncat)
     c = rng.integers(0, 2 ** 64, (ncat, 2), dtype=np.uint64)
     q = rng.integers(0, 2 ** 64, (nq, 2), dtype=np.uint64)
-    q[: nq // 2] = c[rng.integers(0, ncat, nq // 2)] ^ np.uint64(5)
+    q[: nq // 2] = c[rng.integers(0, ncat, nq // 2)] ^ np.uint64(5)  # near duplicates
     _check(q, c, k)
+
+
+def test_query_blocks():
+    # 8192 queries are taken at a time
+    rng = np.random.default_rng(2)
+    c = rng.integers(0, 2 ** 64, (3000, 2), dtype=np.uint64)
+    _check(rng.integers(0, 2 ** 64, (8200, 2), dtype=np.uint64), c, 5)
 
 
 def test_crowded_distances():
