@@ -201,41 +201,61 @@ __global__ void __launch_bounds__(256) votes_kernel(const uint4* __restrict__ q,
 }
 
 // Exact FP32 L2^2 re-rank of each query's k candidates (reference summation
-// order), sorted by (d2, index).  One warp per query.
-__global__ void l2_rerank_kernel(const float* __restrict__ qd, int nq, const float* __restrict__ cd,
-                                 const uint32_t* __restrict__ cand, int k, uint32_t* __restrict__ out_idx,
-                                 float* __restrict__ out_d2) {
-  __shared__ unsigned long long s_keys[8][kTopKMax];
+// order), sorted by (d2, index).  One warp per query; its candidates' rows come into
+// shared memory kRerankRows at a time (a row is one coalesced 512-byte asynchronous
+// copy), where lane c sums candidate c.  Bound by the random 512-byte rows: 4096 x 64 of
+// a 2M-row catalog (134 MB) took 147 us with a lane walking each row in global memory.
+constexpr int kRerankRows = 16;
+constexpr int kRerankStride = 132;  // floats per staged row: lanes of different rows hit distinct banks
+constexpr int kRerankWarps = 8;
+constexpr size_t kRerankSmem = sizeof(float) * kRerankWarps * kRerankRows * kRerankStride;
+__global__ void __launch_bounds__(32 * kRerankWarps) l2_rerank_kernel(const float* __restrict__ qd, int nq,
+                                                                      const float* __restrict__ cd,
+                                                                      const uint32_t* __restrict__ cand, int k,
+                                                                      uint32_t* __restrict__ out_idx,
+                                                                      float* __restrict__ out_d2) {
+  __shared__ unsigned long long s_keys[kRerankWarps][kTopKMax];
+  extern __shared__ float4 s_rows[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int qi = blockIdx.x * 8 + warp;
+  const int qi = blockIdx.x * kRerankWarps + warp;
   if (qi >= nq) return;
   unsigned long long* keys = s_keys[warp];
+  float* rows = reinterpret_cast<float*>(s_rows) + warp * kRerankRows * kRerankStride;
   const float* a = qd + (size_t)qi * 128;
-  for (int t = lane; t < kTopKMax; t += 32) {
-    unsigned long long key = ~0ull;
-    if (t < k) {
-      const uint32_t c = cand[(long long)qi * k + t];
-      if (c != 0xFFFFFFFFu) {
-        const float* b = cd + (size_t)c * 128;
-        float s = 0.0f;
-#pragma unroll 8  // 8 of the row's loads in flight: a lane walks its own row, latency bound
-        for (int i = 0; i < 128; i += 4) {
-          const float4 x = __ldg(reinterpret_cast<const float4*>(a + i));
-          const float4 y = __ldg(reinterpret_cast<const float4*>(b + i));
-          float d = x.x - y.x;
-          s += d * d;
-          d = x.y - y.y;
-          s += d * d;
-          d = x.z - y.z;
-          s += d * d;
-          d = x.w - y.w;
-          s += d * d;
-        }
-        // non-negative floats order like their bit patterns
-        key = ((unsigned long long)__float_as_uint(s) << 32) | c;
-      }
+  for (int t = lane; t < kTopKMax; t += 32) keys[t] = ~0ull;
+  for (int t0 = 0; t0 < k; t0 += kRerankRows) {
+    const int nr = min(kRerankRows, k - t0);
+    const uint32_t mine = lane < nr ? cand[(long long)qi * k + t0 + lane] : 0xFFFFFFFFu;
+    __syncwarp();  // the previous rows are read
+    for (int r = 0; r < nr; ++r) {
+      const uint32_t c = __shfl_sync(0xffffffffu, mine, r);
+      if (c != 0xFFFFFFFFu)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                         (uint32_t)__cvta_generic_to_shared(rows + r * kRerankStride + 4 * lane)),
+                     "l"(cd + (size_t)c * 128 + 4 * lane)
+                     : "memory");
     }
-    keys[t] = key;
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
+    if (mine != 0xFFFFFFFFu) {
+      const float* b = rows + lane * kRerankStride;
+      float s = 0.0f;
+#pragma unroll 8
+      for (int i = 0; i < 128; i += 4) {
+        const float4 x = __ldg(reinterpret_cast<const float4*>(a + i));
+        const float4 y = *reinterpret_cast<const float4*>(b + i);
+        float d = x.x - y.x;
+        s += d * d;
+        d = x.y - y.y;
+        s += d * d;
+        d = x.z - y.z;
+        s += d * d;
+        d = x.w - y.w;
+        s += d * d;
+      }
+      // non-negative floats order like their bit patterns
+      keys[t0 + lane] = ((unsigned long long)__float_as_uint(s) << 32) | mine;
+    }
   }
   __syncwarp();
   for (int kk = 2; kk <= kTopKMax; kk <<= 1) {
@@ -313,7 +333,10 @@ cudaError_t launch_popc_probe(int blocks, int iters, uint32_t* out, cudaStream_t
 cudaError_t launch_l2_rerank(const float* qd, int nq, const float* cd, const uint32_t* cand, int k,
                              uint32_t* out_idx, float* out_d2, cudaStream_t st) {
   if (nq <= 0) return cudaSuccess;
-  l2_rerank_kernel<<<(nq + 7) / 8, 256, 0, st>>>(qd, nq, cd, cand, k, out_idx, out_d2);
+  cudaError_t e = ensure_smem_attr((const void*)l2_rerank_kernel, kRerankSmem);
+  if (e != cudaSuccess) return e;
+  l2_rerank_kernel<<<(nq + kRerankWarps - 1) / kRerankWarps, 32 * kRerankWarps, kRerankSmem, st>>>(qd, nq, cd, cand, k,
+                                                                                                 out_idx, out_d2);
   return cudaGetLastError();
 }
 
