@@ -921,8 +921,7 @@ psift_status psift_catalog_search(psift_catalog* cat, const psift_features* quer
                                      W + 37, nullptr, nullptr});
   }
   if (!verified.empty()) {
-    if ((st = psift_ransac_batch_dev(ctx, sim.data(), (uint32_t)sim.size(), &ropt, 0)) != PSIFT_OK) return st;
-    if ((st = psift_ransac_batch_dev(ctx, hom.data(), (uint32_t)hom.size(), &ropt, 1)) != PSIFT_OK) return st;
+    if ((st = ransac_both_dev(ctx, sim, hom, ropt)) != PSIFT_OK) return st;
     if (own_tracking) {
       psift_ransac_options dopt;
       psift_ransac_options_default(&dopt);

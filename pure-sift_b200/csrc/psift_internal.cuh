@@ -131,6 +131,9 @@ psift_status autotune_match(psift_ctx* ctx, uint32_t n_desc, uint32_t n_pairs, s
 // Statistics of summarize_tracking over the masked matches (ransac_api.cu).
 void tracking_stats(const psift_match* m, uint32_t n, const uint8_t* mask, const float* q_scale,
                     const float* q_ori, const float* t_scale, const float* t_ori, psift_tracking_summary* out);
+// Similarity and homography RANSAC of the same non-empty match lists (ransac_api.cu).
+psift_status ransac_both_dev(psift_ctx* ctx, const std::vector<psift_ransac_job>& sim,
+                             const std::vector<psift_ransac_job>& hom, const psift_ransac_options& opt);
 // CTAs of `func` resident on the whole device at once (occupancy x SMs), cached.
 cudaError_t resident_ctas(const void* func, int threads, size_t smem, int* out);
 // Writes the u8 inputs of images [b, e) of the batch into their device slots

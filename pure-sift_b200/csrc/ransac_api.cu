@@ -29,8 +29,9 @@ void seeds_for(const psift_ransac_options& o, bool homography, uint64_t& s1, uin
   }
 }
 
+// Jobs [0, n_sim) are similarities, the rest homographies.
 psift_status run_batch(psift_ctx* ctx, const psift_ransac_job* jobs, int n, const psift_ransac_options& opt,
-                       bool homography) {
+                       int n_sim) {
   size_t bytes = sizeof(RansacJob) * n + 4096;
   for (int i = 0; i < n; ++i) {
     const size_t m = jobs[i].n;
@@ -40,9 +41,10 @@ psift_status run_batch(psift_ctx* ctx, const psift_ransac_job* jobs, int n, cons
   if (st != PSIFT_OK) return st;
   RansacJob* d_jobs = (RansacJob*)arena_alloc(ctx, sizeof(RansacJob) * n);
   std::vector<RansacJob> hj(n);
-  uint64_t s1, s2;
-  seeds_for(opt, homography, s1, s2);
   for (int i = 0; i < n; ++i) {
+    const bool homography = i >= n_sim;
+    uint64_t s1, s2;
+    seeds_for(opt, homography, s1, s2);
     const psift_ransac_job& J = jobs[i];
     RansacJob& R = hj[i];
     std::memset(&R, 0, sizeof R);
@@ -89,7 +91,7 @@ psift_status estimate_host(psift_ctx* ctx, const psift_match* m, uint32_t n, con
   int* d_out = (int*)(base + align_up(mb, 256) + align_up(n + 1, 256));  // [0] count [1] has [2..3] iters [8..16] model
   if (n) PSIFT_CUDA_TRY(ctx, cudaMemcpyAsync(d_m, m, mb, cudaMemcpyHostToDevice, ctx->stream));
   psift_ransac_job job{d_m, n, d_mask, (float*)(d_out + 8), d_out + 1, (uint32_t*)d_out, nullptr, (uint32_t*)(d_out + 2)};
-  st = run_batch(ctx, &job, 1, *opt, homography);
+  st = run_batch(ctx, &job, 1, *opt, homography ? 0 : 1);
   if (st != PSIFT_OK) return st;
   st = pinned_reserve(ctx, n + 256);
   if (st != PSIFT_OK) return st;
@@ -106,6 +108,21 @@ psift_status estimate_host(psift_ctx* ctx, const psift_match* m, uint32_t n, con
 }
 
 }  // namespace
+
+// The similarity and the homography estimations of the same match lists (both callers
+// want both): one launch when every job gets an SM of its own, so that the two run side
+// by side instead of one after the other.
+psift_status ransac_both_dev(psift_ctx* ctx, const std::vector<psift_ransac_job>& sim,
+                             const std::vector<psift_ransac_job>& hom, const psift_ransac_options& opt) {
+  if (sim.size() + hom.size() <= (size_t)ctx->num_sms) {
+    std::vector<psift_ransac_job> all(sim);
+    all.insert(all.end(), hom.begin(), hom.end());
+    return run_batch(ctx, all.data(), (int)all.size(), opt, (int)sim.size());
+  }
+  const psift_status st = run_batch(ctx, sim.data(), (int)sim.size(), opt, (int)sim.size());
+  return st != PSIFT_OK ? st : run_batch(ctx, hom.data(), (int)hom.size(), opt, 0);
+}
+
 }  // namespace psift
 
 using namespace psift;
@@ -160,7 +177,7 @@ psift_status psift_ransac_batch_dev(psift_ctx* ctx, const psift_ransac_job* jobs
     if (!jobs[i].model || !jobs[i].has_model || !jobs[i].inlier_count || (jobs[i].n && (!jobs[i].matches || !jobs[i].inlier_mask)))
       return set_error(ctx, PSIFT_ERR_INVALID_ARGUMENT, "null pointer in ransac job");
   if (n == 0) return PSIFT_OK;
-  return run_batch(ctx, jobs, (int)n, *opt, homography != 0);
+  return run_batch(ctx, jobs, (int)n, *opt, homography ? 0 : (int)n);
 }
 
 }  // extern "C"

@@ -869,10 +869,7 @@ psift_status psift_stitch_panorama(psift_ctx* ctx, const psift_rgba_image* image
   psift_ransac_options ropt;
   psift_ransac_options_default(&ropt);
   ropt.reproj_threshold = opt->ransac_threshold;
-  if (!sj.empty()) {
-    if ((s = psift_ransac_batch_dev(ctx, sj.data(), (uint32_t)sj.size(), &ropt, 0)) != PSIFT_OK) return s;
-    if ((s = psift_ransac_batch_dev(ctx, hj.data(), (uint32_t)hj.size(), &ropt, 1)) != PSIFT_OK) return s;
-  }
+  if (!sj.empty() && (s = ransac_both_dev(ctx, sj, hj, ropt)) != PSIFT_OK) return s;
   // ---- results to the host
   std::vector<std::vector<uint8_t>> hluma(N);
   for (int i = 0; i < N; ++i) {
