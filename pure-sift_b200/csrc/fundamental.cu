@@ -1,5 +1,5 @@
 // K13: fundamental-matrix LO-RANSAC (normalised 8-point, Sampson distance) on the
-// GPU, one CTA per match set.
+// GPU, one CTA or one cluster of CTAs per match set.
 //
 // Reference (src/geometry.rs): FundamentalRansacOptions (:107-143), mul_mat3 /
 // transpose / det / normalize_frobenius / vector helpers (:145-207),
@@ -25,12 +25,16 @@
 // Results equal the reference's except where libm differs from CUDA's math
 // functions: `hypot` in the point normalisation (glibc's is not correctly
 // rounded), and `cbrt` / `acos` / `cos` in the 7-point solver.
+#include <cooperative_groups.h>
+
 #include <cmath>
 #include <cstring>
 #include <vector>
 
 #include "psift_internal.cuh"
 #include "ransac_common.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace psift {
 namespace {
@@ -42,7 +46,7 @@ struct FundJob {
   int hard_cap, min_iters;
   uint64_t seed;
   double* cdf;    // n
-  double* terms;  // n
+  double* terms;  // n per CTA of the set
   double* pts;    // 4 per match: the ordered inlier list's coordinates, gathered
   float4* xy;     // (query x, query y, target x, target y) per match
   uint8_t* mask;
@@ -600,23 +604,30 @@ __device__ int cubic_roots(double c3, double c2, double c1, double c0, double* r
 
 // A CTA's threads, by the number of match sets of a launch: 256 (two CTAs per SM),
 // or, up to one set per SM, 512: twice the samples fitted and counted per batch in
-// little more time (the fits are latency-bound chains).  48 sets of 2000 to 8000
-// matches, outliers 10 to 60 %: 13.9 against 24.5 ms, with the matches packed to 16
-// bytes and counts that stop once they cannot reach the incumbent's.
+// little more time (the fits are latency-bound chains).  With SMs to spare a set gets a
+// cluster of up to three CTAs: every CTA forms the same samples and replays the same
+// decisions, each fits and counts its share of the batch and hands the counts to the
+// others through distributed shared memory; the first one also does what happens once
+// (sampling CDF, refits, outputs).  48 sets of 2000 to 8000 matches, outliers 10 to
+// 60 %: 24.5 ms with 256 threads and 24-byte match records read, 13.9 with 512, packed
+// matches and counts that stop once they cannot reach the incumbent's, 9.97 with
+// clusters of two.  Sets of 800 matches at 40 %: 4.67 ms with one CTA each (100 sets),
+// 3.35 with two (74), 2.73 with three (44).
 template <int THREADS>
 struct FundCta {
 static constexpr int kFThreads = THREADS;
-static constexpr int kFB = THREADS / 4;  // hypotheses per batch, a quad of lanes each
-static constexpr int kFWin = 32 * kFB;   // resolved draws per window (>= 32 per iteration)
+static constexpr int kFB = THREADS / 4;  // hypotheses per batch and CTA, a quad of lanes each
+static constexpr int kFC = THREADS == 512 ? 3 : 1;  // most CTAs per match set (a cluster)
+static constexpr int kFWin = 32 * kFB;   // resolved draws per window (refilled when a batch needs more)
 static constexpr int kPass = 2;          // hypotheses a warp counts per pass over the matches
 static constexpr int kCheck = 16;        // matches per lane between checks for an early end
 
 struct FShared {
   double F[kFB][9];
-  int samp[kFB][8];
-  int sok[kFB], fok[kFB], cnt[kFB], sdup[kFB];
+  int samp[kFC * kFB][8];
+  int sok[kFC * kFB], fok[kFC * kFB], cnt[kFC * kFB], sdup[kFC * kFB];
   int draws[kFWin];
-  double best[9], cand[9];
+  double best[9], cand[9], tie[9];
   double best_err;
   int best_err_known, best_count, have, max_iters, iter;
   int nb, refill;
@@ -878,52 +889,70 @@ static __device__ void seven_point(const FundJob& J, FShared& S) {
 
 static constexpr size_t kJacSmem = sizeof(double) * 162 * kFB;  // A and V of every sample of a batch
 
-static __device__ void run(const FundJob& J, FShared& S) {
+static __device__ void run(const FundJob& J0, FShared& S) {
   extern __shared__ double jac[];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = (int)cluster.block_rank(), ctas = (int)cluster.num_blocks();
+  FundJob J = J0;
+  J.terms += (size_t)rank * J.n;  // the tie-break's scratch, a row per CTA
   const int n = J.n, t = threadIdx.x;
   if (t == 0) {
-    *J.has_f = 0;
-    *J.count = 0;
-    if (J.iters) *J.iters = 0;
     S.have = 0;
+    if (rank == 0) {
+      *J.has_f = 0;
+      *J.count = 0;
+      if (J.iters) *J.iters = 0;
+    }
   }
-  for (int i = t; i < n; i += kFThreads) {
-    J.mask[i] = 0;
-    const psift_match& a = J.m[i];
-    J.xy[i] = make_float4(a.query_x, a.query_y, a.target_x, a.target_y);
-  }
+  if (rank == 0)
+    for (int i = t; i < n; i += kFThreads) {
+      J.mask[i] = 0;
+      const psift_match& a = J.m[i];
+      J.xy[i] = make_float4(a.query_x, a.query_y, a.target_x, a.target_y);
+    }
   __syncthreads();
-  if (n < 7) return;
+  if (n < 7 || (n == 7 && rank > 0)) return;
   if (n == 7) {
     if (t == 0) seven_point(J, S);
     __syncthreads();
   } else {
-    // build_ratio_weighted_cdf: weights in parallel, the running sum in order
-    for (int i = t; i < n; i += kFThreads) {
-      const float rf = J.m[i].ratio;
-      double r = 1.0;
-      if (isfinite(rf)) r = fmin(fmax((double)rf, 0.05), 1.0);
-      J.cdf[i] = 1.0 / r;
-    }
-    __syncthreads();
-    if (t == 0) {
-      double acc = 0.0;
-      int i = 0;
-      for (; i + kSeqAhead <= n; i += kSeqAhead) {
-        double w[kSeqAhead];
+    if (rank == 0) {
+      // build_ratio_weighted_cdf: weights in parallel, the running sum in order
+      for (int i = t; i < n; i += kFThreads) {
+        const float rf = J.m[i].ratio;
+        double r = 1.0;
+        if (isfinite(rf)) r = fmin(fmax((double)rf, 0.05), 1.0);
+        J.cdf[i] = 1.0 / r;
+      }
+      __syncthreads();
+      if (t == 0) {
+        double acc = 0.0;
+        int i = 0;
+        for (; i + kSeqAhead <= n; i += kSeqAhead) {
+          double w[kSeqAhead];
 #pragma unroll
-        for (int q = 0; q < kSeqAhead; ++q) w[q] = J.cdf[i + q];
+          for (int q = 0; q < kSeqAhead; ++q) w[q] = J.cdf[i + q];
 #pragma unroll
-        for (int q = 0; q < kSeqAhead; ++q) {
-          acc += w[q];
-          J.cdf[i + q] = acc;
+          for (int q = 0; q < kSeqAhead; ++q) {
+            acc += w[q];
+            J.cdf[i + q] = acc;
+          }
         }
+        for (; i < n; ++i) {
+          acc += J.cdf[i];
+          J.cdf[i] = acc;
+        }
+        S.ev_err = acc;
       }
-      for (; i < n; ++i) {
-        acc += J.cdf[i];
-        J.cdf[i] = acc;
+      __syncthreads();
+      if (S.ev_err > 0.0) {
+        const double inv = 1.0 / S.ev_err;
+        for (int i = t; i < n; i += kFThreads) J.cdf[i] *= inv;
       }
-      S.ev_err = acc;
+      __syncthreads();
+      if (t == 0) J.cdf[n - 1] = 1.0;
+    }
+    if (t == 0) {
       S.best_count = 0;
       S.best_err = __longlong_as_double(0x7ff0000000000000ll);
       S.best_err_known = 1;
@@ -932,19 +961,13 @@ static __device__ void run(const FundJob& J, FShared& S) {
       S.tpos = 0;
       S.wb = 0;
     }
-    __syncthreads();
-    if (S.ev_err > 0.0) {
-      const double inv = 1.0 / S.ev_err;
-      for (int i = t; i < n; i += kFThreads) J.cdf[i] *= inv;
-    }
-    __syncthreads();
-    if (t == 0) J.cdf[n - 1] = 1.0;
+    cluster.sync();  // J.xy and J.cdf are complete
     for (int k = t; k < kFWin; k += kFThreads) S.draws[k] = sample_at(J.cdf, n, J.seed, (uint64_t)k);
     __syncthreads();
 
     while (S.iter < S.max_iters) {
       // 1. samples of the next iterations (thread 0 walks the resolved draws)
-      const int want = min(kFB, S.max_iters - S.iter);
+      const int want = min(kFB * ctas, S.max_iters - S.iter);
       if (t == 0) S.nb = 0;
       __syncthreads();
       while (true) {
@@ -1010,13 +1033,16 @@ static __device__ void run(const FundJob& J, FShared& S) {
         __syncthreads();
       }
       const int nb = S.nb;
+      // this CTA's share [h_lo, h_hi) of the batch; S.F is indexed from h_lo
+      const int share = (nb + ctas - 1) / ctas, h_lo = min(rank * share, nb), h_hi = min(h_lo + share, nb);
       // 2. fits, a quad of lanes per sample
       {
-        const int h = t >> 2, ql = t & 3;
+        const int h = h_lo + (t >> 2), ql = t & 3;
         const unsigned qmask = 0xFu << (t & 28);
-        if (h < nb) {
+        if (h < h_hi) {
+          double* A = jac + (t >> 2) * 162;
           bool ok = false;
-          if (S.sok[h]) ok = quad_fit8(J.m, S.samp[h], jac + h * 162, jac + h * 162 + 81, ql, qmask, S.F[h]);
+          if (S.sok[h]) ok = quad_fit8(J.m, S.samp[h], A, A + 81, ql, qmask, S.F[t >> 2]);
           if (ql == 0) S.fok[h] = ok ? 1 : 0;
         }
       }
@@ -1029,18 +1055,18 @@ static __device__ void run(const FundJob& J, FShared& S) {
         // can reach the incumbent's count any more: the replay only asks whether a
         // count is at least that, and it never falls.
         const int best = S.best_count;
-        for (int h0 = warp; h0 < nb; h0 += kPass * (kFThreads / 32)) {
+        for (int h0 = h_lo + warp; h0 < h_hi; h0 += kPass * (kFThreads / 32)) {
           double f[kPass][9];
           bool v[kPass], any = false;
           int c[kPass];
 #pragma unroll
           for (int u = 0; u < kPass; ++u) {
             const int h = h0 + u * (kFThreads / 32);
-            v[u] = h < nb && S.fok[h] != 0;
+            v[u] = h < h_hi && S.fok[h] != 0;
             any |= v[u];
             c[u] = 0;
 #pragma unroll
-            for (int i = 0; i < 9; ++i) f[u][i] = v[u] ? S.F[h][i] : 0.0;
+            for (int i = 0; i < 9; ++i) f[u][i] = v[u] ? S.F[h - h_lo][i] : 0.0;
           }
           for (int i0 = 0; any && i0 < n; i0 += 32 * kCheck) {
             const int i1 = min(i0 + 32 * kCheck, n);
@@ -1059,11 +1085,22 @@ static __device__ void run(const FundJob& J, FShared& S) {
           for (int u = 0; u < kPass; ++u) {
             const int h = h0 + u * (kFThreads / 32);
             const int sum = (int)__reduce_add_sync(0xffffffffu, (unsigned)c[u]);
-            if (lane == 0 && h < nb) S.cnt[h] = sum;
+            if (lane == 0 && h < h_hi) S.cnt[h] = sum;
           }
         }
       }
-      __syncthreads();
+      if (ctas > 1) {  // every CTA replays: hand the others this share's outcome
+        __syncthreads();
+        for (int c = 1; c < ctas; ++c) {
+          FShared* R = cluster.map_shared_rank(&S, (unsigned)((rank + c) % ctas));
+          for (int h = h_lo + t; h < h_hi; h += kFThreads) {
+            R->fok[h] = S.fok[h];
+            R->cnt[h] = S.cnt[h];
+          }
+        }
+      }
+      cluster.sync();
+      auto model = [&](int k) { return cluster.map_shared_rank(&S, (unsigned)(k / share))->F[k % share]; };
       // 4. the reference's decisions, in order
       for (int k = 0; k < nb; ++k) {
         if (t == 0) {
@@ -1076,7 +1113,8 @@ static __device__ void run(const FundJob& J, FShared& S) {
               const int c = S.cnt[k];
               if (c > S.best_count) {
                 S.best_count = c;
-                for (int i = 0; i < 9; ++i) S.best[i] = S.F[k][i];
+                const double* f = model(k);
+                for (int i = 0; i < 9; ++i) S.best[i] = f[i];
                 S.best_err_known = 0;
                 S.have = 1;
                 S.max_iters = adaptive_epipolar(c, n, J.conf, J.min_iters, J.hard_cap);
@@ -1098,18 +1136,21 @@ static __device__ void run(const FundJob& J, FShared& S) {
               S.best_err_known = 1;
             }
           }
-          evaluate(J, S, S.F[k], c, e);
+          if (t < 9) S.tie[t] = model(k)[t];
+          __syncthreads();
+          evaluate(J, S, S.tie, c, e);
           if (t == 0 && e < S.best_err) {
             S.best_err = e;
-            for (int i = 0; i < 9; ++i) S.best[i] = S.F[k][i];
+            for (int i = 0; i < 9; ++i) S.best[i] = S.tie[i];
             S.have = 1;
             S.max_iters = adaptive_epipolar(S.best_count, n, J.conf, J.min_iters, J.hard_cap);
           }
         }
         __syncthreads();  // every thread has read S.act before thread 0 rewrites it
       }
-      __syncthreads();
+      cluster.sync();  // the models and counts of this batch are read
     }
+    if (rank > 0) return;
     if (t == 0 && J.iters) *J.iters = S.iter;
     // 5. LO refits over the ordered inlier list
     if (S.have) {
@@ -1163,16 +1204,53 @@ static __device__ void run(const FundJob& J, FShared& S) {
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS) fundamental_kernel(const FundJob* __restrict__ jobs) {
   __shared__ typename FundCta<THREADS>::FShared S;
-  FundCta<THREADS>::run(jobs[blockIdx.x], S);
+  FundCta<THREADS>::run(jobs[blockIdx.x / cg::this_cluster().num_blocks()], S);
+}
+
+// The CTAs per set in a launch of n sets: the largest cluster up to FundCta::kFC with
+// which all the sets still run at once (a second wave would cost more than it gives).
+template <int THREADS>
+cudaError_t cluster_size(int n, int* out) {
+  *out = 1;
+  for (int c = FundCta<THREADS>::kFC; c > 1; --c) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(n * c));
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = FundCta<THREADS>::kJacSmem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)c;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int fit = 0;
+    const cudaError_t e = cudaOccupancyMaxActiveClusters(&fit, fundamental_kernel<THREADS>, &cfg);
+    if (e != cudaSuccess) return e;
+    if (n <= fit) {
+      *out = c;
+      break;
+    }
+  }
+  return cudaSuccess;
 }
 
 template <int THREADS>
-cudaError_t launch_fundamental(const FundJob* jobs, int n, cudaStream_t st) {
+cudaError_t launch_fundamental(const FundJob* jobs, int n, int ctas, cudaStream_t st) {
   constexpr size_t smem = FundCta<THREADS>::kJacSmem;
   cudaError_t e = ensure_smem_attr((const void*)fundamental_kernel<THREADS>, smem);
   if (e != cudaSuccess) return e;
-  fundamental_kernel<THREADS><<<n, THREADS, smem, st>>>(jobs);
-  return cudaGetLastError();
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(n * ctas));
+  cfg.blockDim = dim3(THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)ctas;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, fundamental_kernel<THREADS>, jobs);
 }
 
 psift_status validate_fundamental_options(psift_ctx* ctx, const psift_fundamental_options* o) {
@@ -1184,10 +1262,20 @@ psift_status validate_fundamental_options(psift_ctx* ctx, const psift_fundamenta
 
 psift_status run_fundamental(psift_ctx* ctx, const psift_fundamental_job* jobs, int n,
                              const psift_fundamental_options& o) {
-  size_t bytes = sizeof(FundJob) * (size_t)n + 4096;
-  for (int i = 0; i < n; ++i) bytes += 64 * (size_t)jobs[i].n + 4 * 256;
-  psift_status st = arena_reserve(ctx, bytes);
-  if (st != PSIFT_OK) return st;
+  int ctas = 1;
+  if (n <= ctx->num_sms) {
+    cudaError_t ce = ensure_smem_attr((const void*)fundamental_kernel<512>, FundCta<512>::kJacSmem);
+    if (ce == cudaSuccess) ce = cluster_size<512>(n, &ctas);
+    if (ce != cudaSuccess) return cuda_error(ctx, ce, "fundamental_ransac");
+  }
+  psift_status st;
+  for (;;) {
+    size_t bytes = sizeof(FundJob) * (size_t)n + 4096;
+    for (int i = 0; i < n; ++i) bytes += (56 + 8 * (size_t)ctas) * (size_t)jobs[i].n + 4 * 256;
+    if ((st = arena_reserve(ctx, bytes)) == PSIFT_OK) break;
+    if (ctas == 1) return st;
+    ctas = 1;  // a row of terms per CTA does not fit: one CTA per set
+  }
   FundJob* d_jobs = (FundJob*)arena_alloc(ctx, sizeof(FundJob) * n);
   std::vector<FundJob> hj(n);
   const double thr = fmax(o.sampson_threshold, 0.25);
@@ -1203,7 +1291,7 @@ psift_status run_fundamental(psift_ctx* ctx, const psift_fundamental_job* jobs, 
     F.min_iters = std::min(64, hard_cap);
     F.seed = o.seed;
     F.cdf = (double*)arena_alloc(ctx, 8 * (size_t)J.n + 8);
-    F.terms = (double*)arena_alloc(ctx, 8 * (size_t)J.n + 8);
+    F.terms = (double*)arena_alloc(ctx, 8 * (size_t)ctas * J.n + 8);
     F.pts = (double*)arena_alloc(ctx, 32 * (size_t)J.n + 32);
     F.xy = (float4*)arena_alloc(ctx, sizeof(float4) * (size_t)J.n + 16);
     F.mask = J.inlier_mask;
@@ -1215,8 +1303,8 @@ psift_status run_fundamental(psift_ctx* ctx, const psift_fundamental_job* jobs, 
   }
   PSIFT_CUDA_TRY(ctx, cudaMemcpyAsync(d_jobs, hj.data(), sizeof(FundJob) * n, cudaMemcpyHostToDevice, ctx->stream));
   StageScope sc(ctx, STAGE_RANSAC);
-  const cudaError_t e = n <= ctx->num_sms ? launch_fundamental<512>(d_jobs, n, ctx->stream)
-                                          : launch_fundamental<256>(d_jobs, n, ctx->stream);
+  const cudaError_t e = n <= ctx->num_sms ? launch_fundamental<512>(d_jobs, n, ctas, ctx->stream)
+                                          : launch_fundamental<256>(d_jobs, n, 1, ctx->stream);
   ctx->launches++;
   if (e != cudaSuccess) return cuda_error(ctx, e, "fundamental_ransac");
   return PSIFT_OK;

@@ -23,3 +23,22 @@ def test_result_does_not_depend_on_the_number_of_sets():
         if f is not None:
             np.testing.assert_array_equal(f, f1)
     ctx.close()
+
+
+@pytest.mark.parametrize("sets", [1, 36, 49, 74, 75, 148])
+def test_result_does_not_depend_on_the_ctas_of_a_set(sets):
+    """Clusters of three, two and one CTA (fewer as the launch holds more sets) against the
+    CTAs of 256 threads of a launch of more sets than SMs."""
+    ctx = psift.Context(0)
+    sizes = [7, 8, 9, 33, 200, 700, 1025]
+    base = [synth.epipolar_matches(n, 0.1 * (k % 8), 900 + k)[0] for k, n in enumerate(sizes)]
+    base.reverse()
+    opt = psift.FundamentalRansacOptions(max_iters=700)
+    many = psift.fundamental_batch((base * 23)[:156], opt, ctx)
+    for i, (mask, f, iters) in enumerate(psift.fundamental_batch((base * 23)[:sets], opt, ctx)):
+        m1, f1, it1 = many[i % len(base)]
+        np.testing.assert_array_equal(mask, m1)
+        assert iters == it1 and (f is None) == (f1 is None)
+        if f is not None:
+            np.testing.assert_array_equal(f, f1)
+    ctx.close()
