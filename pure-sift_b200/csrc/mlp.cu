@@ -6,14 +6,18 @@
 // the forward pass rounds weights and activations to bf16 (round to nearest even)
 // and accumulates in f32.  The backward pass is f32 on the same bf16-rounded
 // operands (straight-through rounding).  Training is deterministic:
-//   mlp_step_kernel    a CTA per chunk of samples: forward, dL/dz for every layer,
+//   mlp_step_kernel    a cluster of CTAs per chunk of samples: forward, dL/dz for every layer,
 //                      per-parameter sums over the chunk's samples in order;
 //   mlp_update_kernel  sums over the chunks in order, Adam update of the f32 masters,
 //                      the minibatch loss.
 // Loss: mean binary cross-entropy over the minibatch.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 
 #include "psift_internal.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace psift {
 
@@ -83,35 +87,55 @@ __global__ void __launch_bounds__(256) mlp_infer_kernel(const float* __restrict_
   }
 }
 
-// One training step's samples, forward and backward, and their gradient sums: a CTA
-// per chunk of kGradChunk samples, everything in shared memory.  The three 128 x 64 x
-// 64 products (layer 2, its transpose, the W2 gradient) are register-tiled: a thread
-// holds 4 x 4 (or 4 x 2) results and takes one step of the inner index at a time, so
-// every result is the same chain of fused multiply-adds, in the same order, as one
-// thread per sample (or per parameter) would compute.  Deterministic: parameter sums
-// run over the chunk's samples in order, the chunks are added in order by
-// mlp_update_kernel.
-// Bound by shared-memory loads and the FP32 pipe (3 x 4096 cycles per chunk): a step
-// of 4096 samples takes 32 CTAs; as separate one-thread-per-sample and
-// one-thread-per-parameter kernels through global memory it was latency bound.
+// One training step's samples, forward and backward, and their gradient sums: a cluster
+// of kStepCtas CTAs per chunk of kGradChunk samples, everything in shared memory.  For
+// the samples' passes each CTA takes a quarter of the chunk; for the sums over the
+// chunk's samples each takes a quarter of the units and fetches its columns of the
+// others' activations and derivatives through distributed shared memory.  The products
+// (layer 2, its transpose, the W2 gradient) are register-tiled: a thread holds 4 x 2
+// results and takes one step of the inner index at a time, so every result is the same
+// chain of fused multiply-adds, in the same order, as one thread per sample (or per
+// parameter) would compute.  Deterministic: parameter sums run over the chunk's samples
+// in order, the chunks are added in order by mlp_update_kernel.
+// Bound by shared-memory loads (a 4 x 2 tile loads 6 values for 8 multiply-adds) and by
+// the latency of the phases, which depend on one another.
+// A step of 4096 samples, its update included: 65.5 us as one-thread-per-sample and
+// one-thread-per-parameter kernels through global memory, 41 with one CTA per chunk, 20.5
+// like this; of 128 samples 61.8 -> 18.5, of 65,536 samples 266 -> 153 us.
 constexpr int kGradChunk = 128;
-constexpr int kStepThreads = 512;
-constexpr int kSS = kGradChunk + 4;  // row stride of [unit][sample] arrays
-constexpr int kHS = kH + 4;          // row stride of [sample][unit] and weight arrays
-constexpr int kXS = kF + 4;          // row stride of the features
+constexpr int kStepCtas = 4;
+constexpr int kStepThreads = 256;
+constexpr int kCtaSamples = kGradChunk / kStepCtas;
+constexpr int kCtaUnits = kH / kStepCtas;
+constexpr int kSS = kCtaSamples + 4;  // row stride of [unit][sample] arrays
+constexpr int kHS = kH + 4;           // row stride of [sample][unit] arrays and of w2
+constexpr int kTS = kH + 2;           // row stride of w2t: two-way conflicts at most in its transposing stores
 
 struct StepSmem {
-  float w2[kH][kHS];    // [j][k]
-  float w2t[kH][kHS];   // [k][j]
-  float t[kH][kSS];     // h1 [k][sample], then dz2 [j][sample]
-  float h1[kGradChunk][kHS];  // activations: +0 where z <= 0, never elsewhere (see relu_bf16)
-  float h2[kGradChunk][kHS];
-  float dz2[kGradChunk][kHS];
-  float dz1[kGradChunk][kHS];
-  float x[kGradChunk][kXS];
+  union {
+    struct {
+      float w2[kH][kHS];   // [j][k]
+      float w2t[kH][kTS];  // [k][j]
+    };
+    float h1_all[kGradChunk][kH];  // after the passes: the chunk's layer-1 activations
+  };
+  union {
+    float t[kH][kSS];  // h1 [k][sample], then dz2 [j][sample]
+    float dz2_all[kGradChunk][kCtaUnits];  // after the passes: this CTA's units, as the next two
+  };
+  float dz1_all[kGradChunk][kCtaUnits];
+  float h2_all[kGradChunk][kCtaUnits];
+  float x_all[kGradChunk][kF];
+  // this CTA's samples; read by the cluster
+  float h1[kCtaSamples][kHS];  // activations: +0 where z <= 0, never elsewhere (see relu_bf16)
+  float h2[kCtaSamples][kHS];
+  float dz2[kCtaSamples][kHS];
+  float dz1[kCtaSamples][kHS];
+  float x[kCtaSamples][kF];
+  float dz3[kCtaSamples];
   float w1[kH][kF];
   float b1[kH], b2[kH], w3[kH];
-  float dz3[kGradChunk];
+  float dz3_all[kGradChunk];
   float b3;
 };
 
@@ -124,19 +148,26 @@ __device__ __forceinline__ float relu_bf16(float z) {
 }
 __device__ __forceinline__ bool active(float h) { return __float_as_uint(h) != 0u; }
 
-__global__ void __launch_bounds__(kStepThreads) mlp_step_kernel(const float* __restrict__ params,
-                                                                const float* __restrict__ X,
-                                                                const float* __restrict__ Y,
-                                                                const int* __restrict__ idx, int B,
-                                                                float* __restrict__ loss_o,
-                                                                float* __restrict__ partial) {
+__global__ void __cluster_dims__(kStepCtas, 1, 1) __launch_bounds__(kStepThreads, 2)
+    mlp_step_kernel(const float* __restrict__ params, const float* __restrict__ X, const float* __restrict__ Y,
+                    const int* __restrict__ idx, int B, float* __restrict__ loss_o, float* __restrict__ partial) {
   extern __shared__ __align__(16) uint8_t step_smem[];
   StepSmem& s = *reinterpret_cast<StepSmem*>(step_smem);
-  const int tid = threadIdx.x;
-  const int b0 = blockIdx.x * kGradChunk, nb = min(kGradChunk, B - b0);
-  // parameters (weights rounded to bf16) and the chunk's features
+  cg::cluster_group cluster = cg::this_cluster();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int rank = (int)cluster.block_rank(), chunk = blockIdx.x / kStepCtas;
+  const int nb = min(kGradChunk, B - chunk * kGradChunk);             // the chunk's samples
+  const int s0 = chunk * kGradChunk + rank * kCtaSamples;             // this CTA's first
+  const int ns = min(kCtaSamples, max(nb - rank * kCtaSamples, 0));   // and how many (the rest count as zeros)
+  {  // features, a value per thread
+    const int r = tid / kF, k = tid % kF;
+    s.x[r][k] = r < ns ? bf16r(X[(size_t)(idx ? idx[s0 + r] : s0 + r) * kF + k]) : 0.0f;
+  }
+  // parameters, the weights rounded to bf16
   for (int i = tid; i < kH * kF; i += kStepThreads) (&s.w1[0][0])[i] = bf16r(params[kOffW1 + i]);
-  for (int i = tid; i < kH * kH; i += kStepThreads) {
+#pragma unroll
+  for (int q = 0; q < kH * kH / kStepThreads; ++q) {
+    const int i = tid + q * kStepThreads;
     const float w = bf16r(params[kOffW2 + i]);
     s.w2[i / kH][i % kH] = w;
     s.w2t[i % kH][i / kH] = w;
@@ -147,52 +178,54 @@ __global__ void __launch_bounds__(kStepThreads) mlp_step_kernel(const float* __r
     s.w3[tid] = bf16r(params[kOffW3 + tid]);
   }
   if (tid == 0) s.b3 = params[kOffB3];
-  for (int i = tid; i < kGradChunk * kF; i += kStepThreads) {
-    const int r = i / kF, k = i % kF;
-    s.x[r][k] = r < nb ? bf16r(X[(size_t)(idx ? idx[b0 + r] : b0 + r) * kF + k]) : 0.0f;
-  }
   __syncthreads();
-  // layer 1: a warp shares the unit j, lanes are samples
-  for (int i = tid; i < kGradChunk * kH; i += kStepThreads) {
-    const int r = i % kGradChunk, j = i / kGradChunk;
-    float z = s.b1[j];
+  const int v0 = 8 * warp;  // lane: a sample, warp: 8 units
+  {                         // layer 1
+    float x[kF], h[8];
 #pragma unroll
-    for (int k = 0; k < kF; ++k) z = __fmaf_rn(s.w1[j][k], s.x[r][k], z);
-    const float h = relu_bf16(z);
-    s.t[j][r] = h;
-    s.h1[r][j] = h;
-  }
-  __syncthreads();
-  // 4 x 4 tiles: a warp covers 32 samples x 16 units, lanes 8 x 4 tiles (two
-  // conflict-free 128-bit loads per step)
-  const int lane = tid & 31, warp = tid >> 5;
-  const int r0 = 32 * (warp & 3) + 4 * (lane & 7), u0 = 16 * (warp >> 2) + 4 * (lane >> 3);
-  {  // layer 2
-    float acc[4][4];
+    for (int k = 0; k < kF; ++k) x[k] = s.x[lane][k];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int q = 0; q < 8; ++q) {
+      float z = s.b1[v0 + q];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = s.b2[u0 + j];
-#pragma unroll 4
-    for (int k = 0; k < kH; ++k) {
-      const float4 h = *reinterpret_cast<const float4*>(&s.t[k][r0]), w = *reinterpret_cast<const float4*>(&s.w2t[k][u0]);
-      const float hv[4] = {h.x, h.y, h.z, h.w}, wv[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = __fmaf_rn(wv[j], hv[i], acc[i][j]);
+      for (int k = 0; k < kF; ++k) z = __fmaf_rn(s.w1[v0 + q][k], x[k], z);
+      h[q] = relu_bf16(z);
+      s.t[v0 + q][lane] = h[q];
     }
+    *reinterpret_cast<float4*>(&s.h1[lane][v0]) = make_float4(h[0], h[1], h[2], h[3]);
+    *reinterpret_cast<float4*>(&s.h1[lane][v0 + 4]) = make_float4(h[4], h[5], h[6], h[7]);
+  }
+  __syncthreads();
+  // 4 (samples) x 2 (units) tiles: a warp covers the 32 samples x 8 units, lanes 8 x 4
+  // tiles (two loads without conflicts per step)
+  const int r0 = 4 * (lane & 7), u0 = 8 * warp + 2 * (lane >> 3);
+  {  // layer 2
+    float acc[4][2];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      *reinterpret_cast<float4*>(&s.h2[r0 + i][u0]) =
-          make_float4(relu_bf16(acc[i][0]), relu_bf16(acc[i][1]), relu_bf16(acc[i][2]), relu_bf16(acc[i][3]));
+      acc[i][0] = s.b2[u0];
+      acc[i][1] = s.b2[u0 + 1];
     }
+#pragma unroll 8
+    for (int k = 0; k < kH; ++k) {
+      const float4 h = *reinterpret_cast<const float4*>(&s.t[k][r0]);
+      const float2 w = *reinterpret_cast<const float2*>(&s.w2t[k][u0]);
+      const float hv[4] = {h.x, h.y, h.z, h.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        acc[i][0] = __fmaf_rn(w.x, hv[i], acc[i][0]);
+        acc[i][1] = __fmaf_rn(w.y, hv[i], acc[i][1]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      *reinterpret_cast<float2*>(&s.h2[r0 + i][u0]) = make_float2(relu_bf16(acc[i][0]), relu_bf16(acc[i][1]));
   }
   __syncthreads();
   // layer 3, loss and its derivative: a thread per sample
-  if (tid < kGradChunk) {
+  if (tid < kCtaSamples) {
     float z3 = s.b3;
-#pragma unroll 4
+#pragma unroll
     for (int j = 0; j < kH; j += 4) {
       const float4 h = *reinterpret_cast<const float4*>(&s.h2[tid][j]);
       z3 = __fmaf_rn(s.w3[j], h.x, z3);
@@ -201,50 +234,82 @@ __global__ void __launch_bounds__(kStepThreads) mlp_step_kernel(const float* __r
       z3 = __fmaf_rn(s.w3[j + 3], h.w, z3);
     }
     float dz3 = 0.0f;
-    if (tid < nb) {
-      const float y = Y[idx ? idx[b0 + tid] : b0 + tid];
+    if (tid < ns) {
+      const float y = Y[idx ? idx[s0 + tid] : s0 + tid];
       const float p = sigmoidf_(z3);
       // BCE with logits: softplus(z) - y z, numerically stable form
-      loss_o[b0 + tid] = fmaxf(z3, 0.0f) - z3 * y + log1pf(expf(-fabsf(z3)));
+      loss_o[s0 + tid] = fmaxf(z3, 0.0f) - z3 * y + log1pf(expf(-fabsf(z3)));
       dz3 = (p - y) * (1.0f / (float)B);
     }
     s.dz3[tid] = dz3;
   }
   __syncthreads();
-  for (int i = tid; i < kGradChunk * kH; i += kStepThreads) {
-    const int r = i % kGradChunk, j = i / kGradChunk;
-    const float d = active(s.h2[r][j]) ? s.dz3[r] * s.w3[j] : 0.0f;
-    s.t[j][r] = d;
-    s.dz2[r][j] = d;
+  {
+    const float4 ha = *reinterpret_cast<const float4*>(&s.h2[lane][v0]), hb = *reinterpret_cast<const float4*>(&s.h2[lane][v0 + 4]);
+    const float h[8] = {ha.x, ha.y, ha.z, ha.w, hb.x, hb.y, hb.z, hb.w};
+    const float dz3 = s.dz3[lane];
+    float d[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      d[q] = active(h[q]) ? dz3 * s.w3[v0 + q] : 0.0f;
+      s.t[v0 + q][lane] = d[q];
+    }
+    *reinterpret_cast<float4*>(&s.dz2[lane][v0]) = make_float4(d[0], d[1], d[2], d[3]);
+    *reinterpret_cast<float4*>(&s.dz2[lane][v0 + 4]) = make_float4(d[4], d[5], d[6], d[7]);
   }
   __syncthreads();
   {  // back through layer 2
-    float acc[4][4] = {};
-#pragma unroll 4
+    float acc[4][2] = {};
+#pragma unroll 8
     for (int j = 0; j < kH; ++j) {
-      const float4 d = *reinterpret_cast<const float4*>(&s.t[j][r0]), w = *reinterpret_cast<const float4*>(&s.w2[j][u0]);
-      const float dv[4] = {d.x, d.y, d.z, d.w}, wv[4] = {w.x, w.y, w.z, w.w};
+      const float4 d = *reinterpret_cast<const float4*>(&s.t[j][r0]);
+      const float2 w = *reinterpret_cast<const float2*>(&s.w2[j][u0]);
+      const float dv[4] = {d.x, d.y, d.z, d.w};
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int k = 0; k < 4; ++k) acc[i][k] = __fmaf_rn(wv[k], dv[i], acc[i][k]);
+      for (int i = 0; i < 4; ++i) {
+        acc[i][0] = __fmaf_rn(w.x, dv[i], acc[i][0]);
+        acc[i][1] = __fmaf_rn(w.y, dv[i], acc[i][1]);
+      }
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-#pragma unroll
-      for (int k = 0; k < 4; ++k) acc[i][k] = active(s.h1[r0 + i][u0 + k]) ? acc[i][k] : 0.0f;
-      *reinterpret_cast<float4*>(&s.dz1[r0 + i][u0]) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+      const float2 h = *reinterpret_cast<const float2*>(&s.h1[r0 + i][u0]);
+      *reinterpret_cast<float2*>(&s.dz1[r0 + i][u0]) =
+          make_float2(active(h.x) ? acc[i][0] : 0.0f, active(h.y) ? acc[i][1] : 0.0f);
     }
   }
-  __syncthreads();
-  float* part = partial + (size_t)blockIdx.x * kNP;
-  {  // W2 gradient: 4 (j) x 2 (k) per thread, lanes 4 x 8 tiles
-    const int j0 = 16 * (warp & 3) + 4 * (lane & 3), k0 = 16 * (warp >> 2) + 2 * (lane >> 2);
+  cluster.sync();
+  // the chunk's layer-1 activations and features, and this CTA's units of the rest
+  const int c0 = kCtaUnits * rank;
+#pragma unroll
+  for (int q = 0; q < kGradChunk * kH / 4 / kStepThreads; ++q) {
+    const int i = tid + q * kStepThreads, b = i / (kH / 4), c = 4 * (i % (kH / 4));
+    const StepSmem* o = cluster.map_shared_rank(&s, (unsigned)(b / kCtaSamples));
+    *reinterpret_cast<float4*>(&s.h1_all[b][c]) = *reinterpret_cast<const float4*>(&o->h1[b % kCtaSamples][c]);
+  }
+#pragma unroll
+  for (int q = 0; q < kGradChunk * kCtaUnits / 4 / kStepThreads; ++q) {
+    const int i = tid + q * kStepThreads, b = i / (kCtaUnits / 4), c = 4 * (i % (kCtaUnits / 4)), r = b % kCtaSamples;
+    const StepSmem* o = cluster.map_shared_rank(&s, (unsigned)(b / kCtaSamples));
+    *reinterpret_cast<float4*>(&s.dz2_all[b][c]) = *reinterpret_cast<const float4*>(&o->dz2[r][c0 + c]);
+    *reinterpret_cast<float4*>(&s.dz1_all[b][c]) = *reinterpret_cast<const float4*>(&o->dz1[r][c0 + c]);
+    *reinterpret_cast<float4*>(&s.h2_all[b][c]) = *reinterpret_cast<const float4*>(&o->h2[r][c0 + c]);
+  }
+  {
+    const int b = tid / 2, c = 4 * (tid % 2);
+    const StepSmem* o = cluster.map_shared_rank(&s, (unsigned)(b / kCtaSamples));
+    *reinterpret_cast<float4*>(&s.x_all[b][c]) = *reinterpret_cast<const float4*>(&o->x[b % kCtaSamples][c]);
+    if (c == 0) s.dz3_all[b] = o->dz3[b % kCtaSamples];
+  }
+  cluster.sync();  // also: nobody reads this CTA's arrays any more
+  float* part = partial + (size_t)chunk * kNP;
+  if (warp < 4) {  // W2: 4 (j) x 2 (k) per thread, lanes 4 x 8 tiles
+    const int j0 = 4 * (lane & 3), k0 = 16 * warp + 2 * (lane >> 2);
     float acc[4][2] = {};
-#pragma unroll 4
+#pragma unroll 8
     for (int b = 0; b < nb; ++b) {
-      const float4 d = *reinterpret_cast<const float4*>(&s.dz2[b][j0]);
-      const float2 h = *reinterpret_cast<const float2*>(&s.h1[b][k0]);
+      const float4 d = *reinterpret_cast<const float4*>(&s.dz2_all[b][j0]);
+      const float2 h = *reinterpret_cast<const float2*>(&s.h1_all[b][k0]);
       const float dv[4] = {d.x, d.y, d.z, d.w};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -255,40 +320,44 @@ __global__ void __launch_bounds__(kStepThreads) mlp_step_kernel(const float* __r
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
-      for (int k = 0; k < 2; ++k) part[kOffW2 + (j0 + j) * kH + k0 + k] = acc[j][k];
-  }
-  {  // W1 gradient: a parameter per thread
-    const int j = tid / kF, k = tid % kF;
+      for (int k = 0; k < 2; ++k) part[kOffW2 + (c0 + j0 + j) * kH + k0 + k] = acc[j][k];
+  } else if (warp < 6) {  // W1: 1 (j) x 2 (k)
+    const int j = (tid - 128) / (kF / 2), k = 2 * (tid % (kF / 2));
+    float g0 = 0.0f, g1 = 0.0f;
+#pragma unroll 8
+    for (int b = 0; b < nb; ++b) {
+      const float d = s.dz1_all[b][j];
+      const float2 x = *reinterpret_cast<const float2*>(&s.x_all[b][k]);
+      g0 = __fmaf_rn(d, x.x, g0);
+      g1 = __fmaf_rn(d, x.y, g1);
+    }
+    part[kOffW1 + (c0 + j) * kF + k] = g0;
+    part[kOffW1 + (c0 + j) * kF + k + 1] = g1;
+  } else {  // biases and W3
+    const int q = tid - 192, j = q % kCtaUnits;
     float g = 0.0f;
+    if (q < kCtaUnits) {
 #pragma unroll 8
-    for (int b = 0; b < nb; ++b) g = __fmaf_rn(s.dz1[b][j], s.x[b][k], g);
-    part[kOffW1 + tid] = g;
-  }
-  // biases and W3
-  if (tid < 3 * kH + 1) {
-    const int j = tid % kH;
-    float g = 0.0f;
-    if (tid < kH) {
+      for (int b = 0; b < nb; ++b) g += s.dz1_all[b][j];
+      part[kOffB1 + c0 + j] = g;
+    } else if (q < 2 * kCtaUnits) {
 #pragma unroll 8
-      for (int b = 0; b < nb; ++b) g += s.dz1[b][j];
-      part[kOffB1 + j] = g;
-    } else if (tid < 2 * kH) {
+      for (int b = 0; b < nb; ++b) g += s.dz2_all[b][j];
+      part[kOffB2 + c0 + j] = g;
+    } else if (q < 3 * kCtaUnits) {
 #pragma unroll 8
-      for (int b = 0; b < nb; ++b) g += s.dz2[b][j];
-      part[kOffB2 + j] = g;
-    } else if (tid < 3 * kH) {
+      for (int b = 0; b < nb; ++b) g = __fmaf_rn(s.dz3_all[b], s.h2_all[b][j], g);
+      part[kOffW3 + c0 + j] = g;
+    } else if (q == 3 * kCtaUnits && rank == 0) {
 #pragma unroll 8
-      for (int b = 0; b < nb; ++b) g = __fmaf_rn(s.dz3[b], s.h2[b][j], g);
-      part[kOffW3 + j] = g;
-    } else {
-#pragma unroll 8
-      for (int b = 0; b < nb; ++b) g += s.dz3[b];
+      for (int b = 0; b < nb; ++b) g += s.dz3_all[b];
       part[kOffB3] = g;
     }
   }
 }
-static_assert(sizeof(StepSmem) <= 227 * 1024, "one chunk per SM");
-static_assert(kStepThreads == kH * kF && kGradChunk * kH == 16 * kStepThreads, "tiles cover the chunk");
+static_assert(2 * (sizeof(StepSmem) + 1024) <= 228 * 1024, "two CTAs per SM");
+static_assert(kCtaSamples == 32 && kCtaUnits == 16 && kStepThreads == kCtaSamples * kF && kH == 8 * (kStepThreads / 32),
+              "tiles cover the chunk");
 
 // Adds the chunks' gradient sums in chunk order and, with `update`, takes the Adam step
 // on the f32 masters; the last CTA writes the mean of the per-sample losses, in a fixed
@@ -303,6 +372,7 @@ __global__ void __launch_bounds__(kUpdateThreads) mlp_update_kernel(
   if (blockIdx.x == gridDim.x - 1) {
     if (!loss_out) return;
     float sum = 0.0f;
+#pragma unroll 16
     for (int b = t; b < B; b += kUpdateThreads) sum += l[b];
     part[t] = sum;
     __syncthreads();
@@ -316,7 +386,7 @@ __global__ void __launch_bounds__(kUpdateThreads) mlp_update_kernel(
   const int p = blockIdx.x * kUpdateThreads + t;
   if (p >= kNP) return;
   float g = 0.0f;
-#pragma unroll 8
+#pragma unroll 16
   for (int c = 0; c < chunks; ++c) g += partial[(size_t)c * kNP + p];
   grad[p] = g;
   if (update) {
@@ -541,7 +611,7 @@ cudaError_t launch_mlp_step(float* params, const float* X, const float* Y, const
   const int chunks = (B + kGradChunk - 1) / kGradChunk;
   cudaError_t e = ensure_smem_attr((const void*)mlp_step_kernel, sizeof(StepSmem));
   if (e != cudaSuccess) return e;
-  mlp_step_kernel<<<chunks, kStepThreads, sizeof(StepSmem), st>>>(params, X, Y, idx, B, lb, partial);
+  mlp_step_kernel<<<chunks * kStepCtas, kStepThreads, sizeof(StepSmem), st>>>(params, X, Y, idx, B, lb, partial);
   const float b1 = 0.9f, b2 = 0.999f;
   const float bc1 = 1.0f - powf(b1, (float)t), bc2 = 1.0f - powf(b2, (float)t);
   mlp_update_kernel<<<(kNP + kUpdateThreads - 1) / kUpdateThreads + 1, kUpdateThreads, 0, st>>>(
