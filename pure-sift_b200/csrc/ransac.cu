@@ -35,6 +35,41 @@
 
 namespace psift {
 
+template <int N>
+struct Int {
+  static constexpr int value = N;
+};
+
+// ---- packed f32x2
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 r;
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
+      "fma.rn.f32x2 z, x, y, z;\n\tmov.b64 {%0, %1}, z;\n\t}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return r;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 r;
+  asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
+      "mul.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 r;
+  asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
+      "add.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+
+// Offsets i * 9 + j, i < j, of a 9 x 9 matrix's strict upper triangle.
+static __constant__ uint8_t kStrictUpper[36] = {1,  2,  3,  4,  5,  6,  7,  8,  11, 12, 13, 14, 15, 16, 17, 21, 22, 23,
+                                                24, 25, 26, 31, 32, 33, 34, 35, 41, 42, 43, 44, 51, 52, 53, 61, 62, 71};
+
 // A CTA's threads, by the number of match sets of a launch.  The serial parts (replay,
 // sequential sums, the Jacobi of a refit) leave most of a CTA idle, so many sets
 // share the SMs best as four CTAs of 128 threads each (128 registers, ~51 KB of
@@ -56,6 +91,10 @@ static constexpr size_t kJacSmem = sizeof(double) * 162 * kBatch;
 static constexpr int kRowChunk = (int)(kJacSmem / (sizeof(double) * 10));
 // sequential sums over an inlier list stage its points (float4) there
 static constexpr int kPtChunk = (int)(kJacSmem / sizeof(float4));
+// and the counts the first matches' coordinates, as four float arrays of kStage; the
+// last eighth is left to ordered_sum, which breaks ties while they are staged
+static constexpr size_t kSumOff = kJacSmem / 8 * 7 / 16 * 16;
+static constexpr int kStage = (int)(kSumOff / sizeof(float4)) / 64 * 64;
 
 struct RShared {
   int n;
@@ -65,6 +104,9 @@ struct RShared {
   // batch of hypotheses
   float ha[kBatch], hb[kBatch], htx[kBatch], hty[kBatch];
   double H[kBatch][9];
+  float4 hband[kBatch];  // the f32 test's bounds (see h_band)
+  double BH[9], Hc[9];   // the incumbent homography, the candidate being refined
+  unsigned coord_max[3];  // bits of max |query x|, |query y|, |target x or y| over the matches
   int hvalid[kBatch];
   int hcnt[kBatch];
   int quad[kBatch][4];
@@ -74,7 +116,7 @@ struct RShared {
   float fres[8];
   double dres[16];
   double ata[9][9];
-  int draw_ptr, draws_ready;
+  int draw_ptr, draws_ready, dup;
   int draws_s[2 * kDrawChunk];  // draw t lives at [t % (2 * kDrawChunk)]
   int sim_count;
   float sim_model[6];
@@ -197,8 +239,8 @@ static __device__ int adaptive_iters_w(double w, int ss, int min_it, int cap) {
 }
 
 // Sequential sum, in match order, of term(i) for i < n: the CTA computes the
-// terms of a chunk into shared memory (the batch's Jacobi space, free whenever a
-// sum is taken), thread 0 adds them in order with its loads issued ahead of the
+// terms of a chunk into shared memory (the end of the batch's Jacobi space, free
+// whenever a sum is taken), thread 0 adds them in order with its loads issued ahead of the
 // dependent additions; the result is returned to every thread.  Terms of matches
 // that are not inliers are zero, which leaves the running sum unchanged (x + 0 ==
 // x for the finite, non-negative partial sums), so this equals the reference's
@@ -206,8 +248,8 @@ static __device__ int adaptive_iters_w(double w, int ss, int min_it, int cap) {
 template <typename T, typename Term>
 static __device__ T ordered_sum(RShared& S, int n, Term term) {
   extern __shared__ double jac[];
-  T* buf = reinterpret_cast<T*>(jac);
-  constexpr int cap = (int)(kJacSmem / sizeof(T));
+  T* buf = reinterpret_cast<T*>(reinterpret_cast<uint8_t*>(jac) + kSumOff);
+  constexpr int cap = (int)((kJacSmem - kSumOff) / sizeof(T));
   T s = T(0);
   for (int c0 = 0; c0 < n; c0 += cap) {
     const int cn = min(cap, n - c0);
@@ -244,45 +286,105 @@ static __device__ __forceinline__ bool sim_inlier(const float4 p, float a, float
   return e <= tsq;
 }
 
-// A warp's two hypotheses, counted so far to c1 and c2 (per lane) with `rest` matches
-// to go: whether either can still reach `best`, the incumbent's count.  The replay
-// only asks whether a count is at least that, and the incumbent's never falls, so a
-// count may stop short once it cannot.
+// Whether a warp's hypothesis, counted so far to c (per lane) with `rest` matches to go,
+// can still reach `best`, the incumbent's count.  The replay only asks whether a count
+// is at least that, and the incumbent's never falls, so a count may stop short once it
+// cannot.
 static constexpr int kCheck = 16;  // matches per lane between checks
-static __device__ __forceinline__ bool can_reach(bool v1, int c1, bool v2, int c2, int rest, int best) {
-  const int s1 = (int)__reduce_add_sync(0xffffffffu, (unsigned)c1), s2 = (int)__reduce_add_sync(0xffffffffu, (unsigned)c2);
-  return (v1 && s1 + rest >= best) || (v2 && s2 + rest >= best);
+static __device__ __forceinline__ bool can_reach(bool valid, int c, int rest, int best) {
+  const int s = (int)__reduce_add_sync(0xffffffffu, (unsigned)c);
+  return valid && s + rest >= best;
+}
+
+// The first matches' coordinates to shared memory, as four arrays: a lane then reads
+// two matches as packed pairs, and 16 warps re-reading every match for every pass
+// don't go through L2.  Returns how many are staged (a multiple of 64).
+static __device__ int stage_coords(const RansacJob& J, RShared& S) {
+  extern __shared__ double jac[];
+  float* c = reinterpret_cast<float*>(jac);
+  const int ns = min(S.n / 64 * 64, kStage);
+  for (int i = threadIdx.x; i < ns; i += kRThreads) {
+    const float4 p = J.xy[i];
+    c[i] = p.x;
+    c[kStage + i] = p.y;
+    c[2 * kStage + i] = p.z;
+    c[3 * kStage + i] = p.w;
+  }
+  __syncthreads();
+  return ns;
 }
 
 // Inlier counts of the similarity hypotheses h < nh of the batch (S.ha.. /
-// S.hvalid -> S.hcnt): warp w takes h = w, w + 8, ..., two per pass over the
-// matches.  Ends with a block barrier.
-static __device__ void sim_count_batch(const RansacJob& J, RShared& S, int nh, int best) {
+// S.hvalid -> S.hcnt): warp w takes h = w, w + kRWarps, ..., four per pass over the
+// matches.  The staged ones (ns) are taken two per lane in packed arithmetic, with the
+// roundings of sim_inlier: `one` = 1 comes from the kernel's parameters, so that no
+// multiplication and addition become one operation.  Ends with a block barrier.
+// 1000 hypotheses on 5650 matches: 1.71 M cycles with the coordinates read from L2 and
+// scalar arithmetic, 1.18 M like this.
+static __device__ void sim_count_batch(const RansacJob& J, RShared& S, int nh, int best, int ns, float one) {
+  extern __shared__ double jac[];
+  const float* xs = reinterpret_cast<const float*>(jac);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const float tsq = S.tsq_f;
-  for (int h = warp; h < nh; h += 2 * kRWarps) {
-    const int h2 = h + kRWarps;
-    const bool v1 = S.hvalid[h] != 0, v2 = h2 < nh && S.hvalid[h2] != 0;
-    int c1 = 0, c2 = 0;
-    const float a1 = S.ha[h], b1 = S.hb[h], x1 = S.htx[h], y1 = S.hty[h];
-    const float a2 = v2 ? S.ha[h2] : 0.f, b2 = v2 ? S.hb[h2] : 0.f, x2 = v2 ? S.htx[h2] : 0.f,
-                y2 = v2 ? S.hty[h2] : 0.f;
-    bool go = v1 || v2;
-    for (int i0 = 0; go && i0 < S.n; i0 += 32 * kCheck) {
+  const float2 p1 = make_float2(one, one), m1 = make_float2(-one, -one);
+  constexpr int kPass = 4;
+  for (int h0 = warp; h0 < nh; h0 += kPass * kRWarps) {
+    float2 a[kPass], b[kPass], tx[kPass], ty[kPass];
+    bool v[kPass], go = false;
+    int c[kPass];
+#pragma unroll
+    for (int u = 0; u < kPass; ++u) {
+      const int h = h0 + u * kRWarps;
+      v[u] = h < nh && S.hvalid[h] != 0;
+      const float av = v[u] ? S.ha[h] : 0.0f, bv = v[u] ? S.hb[h] : 0.0f;
+      const float xv = v[u] ? S.htx[h] : 0.0f, yv = v[u] ? S.hty[h] : 0.0f;
+      a[u] = make_float2(av, av);
+      b[u] = make_float2(bv, bv);
+      tx[u] = make_float2(xv, xv);
+      ty[u] = make_float2(yv, yv);
+      c[u] = 0;
+      go |= v[u];
+    }
+    auto reach = [&](int rest) {
+      bool any = false;
+#pragma unroll
+      for (int u = 0; u < kPass; ++u) any |= can_reach(v[u], c[u], rest, best);
+      return any;
+    };
+    for (int i0 = 0; go && i0 < ns; i0 += 32 * kCheck) {
+      const int i1 = min(i0 + 32 * kCheck, ns);
+#pragma unroll 2
+      for (int i = i0 + 2 * lane; i < i1; i += 64) {
+        const float2 x = *reinterpret_cast<const float2*>(xs + i), y = *reinterpret_cast<const float2*>(xs + kStage + i);
+        const float2 z = *reinterpret_cast<const float2*>(xs + 2 * kStage + i), w = *reinterpret_cast<const float2*>(xs + 3 * kStage + i);
+#pragma unroll
+        for (int u = 0; u < kPass; ++u) {
+          const float2 dx = fma2(z, m1, add2(fma2(mul2(b[u], y), m1, mul2(a[u], x)), tx[u]));
+          const float2 dy = fma2(w, m1, add2(fma2(mul2(b[u], x), p1, mul2(a[u], y)), ty[u]));
+          const float2 e = fma2(mul2(dx, dx), p1, mul2(dy, dy));
+          c[u] += e.x <= tsq ? 1 : 0;
+          c[u] += e.y <= tsq ? 1 : 0;
+        }
+      }
+      go = reach(S.n - i1);
+    }
+    for (int i0 = ns; go && i0 < S.n; i0 += 32 * kCheck) {
       const int i1 = min(i0 + 32 * kCheck, S.n);
       for (int i = i0 + lane; i < i1; i += 32) {
         const float4 p = J.xy[i];
-        float e;
-        c1 += (v1 && sim_inlier(p, a1, b1, x1, y1, tsq, e)) ? 1 : 0;
-        c2 += (v2 && sim_inlier(p, a2, b2, x2, y2, tsq, e)) ? 1 : 0;
+#pragma unroll
+        for (int u = 0; u < kPass; ++u) {
+          float e;
+          c[u] += sim_inlier(p, a[u].x, b[u].x, tx[u].x, ty[u].x, tsq, e) ? 1 : 0;
+        }
       }
-      go = can_reach(v1, c1, v2, c2, S.n - i1, best);
+      go = reach(S.n - i1);
     }
-    c1 = (int)__reduce_add_sync(0xffffffffu, (unsigned)c1);
-    c2 = (int)__reduce_add_sync(0xffffffffu, (unsigned)c2);
-    if (lane == 0) {
-      S.hcnt[h] = c1;
-      if (h2 < nh) S.hcnt[h2] = c2;
+#pragma unroll
+    for (int u = 0; u < kPass; ++u) {
+      const int h = h0 + u * kRWarps;
+      const int sum = (int)__reduce_add_sync(0xffffffffu, (unsigned)c[u]);
+      if (lane == 0 && h < nh) S.hcnt[h] = sum;
     }
   }
   __syncthreads();
@@ -467,7 +569,8 @@ static __device__ bool sim_consider(const RansacJob& J, RShared& S, SimBest& B, 
 
 // filter_matches_ransac_with_seed (src/pipeline.rs:2055-2191).  Writes the
 // inlier list (J.list, length S.sim_count) and S.sim_model / S.has_sim.
-static __device__ void similarity_ransac(const RansacJob& J, RShared& S, double* jac, uint64_t seed, float thr) {
+static __device__ void similarity_ransac(const RansacJob& J, RShared& S, double* jac, uint64_t seed, float thr,
+                                         float one) {
   const int n = S.n;
   if (threadIdx.x == 0) {
     S.has_sim = 0;
@@ -534,8 +637,8 @@ static __device__ void similarity_ransac(const RansacJob& J, RShared& S, double*
     S.hty[threadIdx.x] = mr.displacement_y;
     S.hvalid[threadIdx.x] = 1;
   }
-  __syncthreads();
-  sim_count_batch(J, S, ntop, 0);
+  const int ns = stage_coords(J, S);  // also: the batch is complete
+  sim_count_batch(J, S, ntop, 0, ns, one);
   SimBest B{1.0f, 0.0f, S.htx[0], S.hty[0], S.hcnt[0], 0.0f, false};
   for (int r = 0; r < ntop; ++r) sim_consider(J, S, B, r);
   __syncthreads();  // the batch slots are rewritten below
@@ -580,7 +683,7 @@ static __device__ void similarity_ransac(const RansacJob& J, RShared& S, double*
       S.hvalid[t] = valid;
     }
     __syncthreads();
-    sim_count_batch(J, S, nh, B.count);
+    sim_count_batch(J, S, nh, B.count, ns, one);
     // replay in order
     for (int h = 0; h < nh; ++h) {
       const int it = base + h;
@@ -642,43 +745,125 @@ static __device__ __forceinline__ bool h_inlier(const float4 p, const double* H,
   return e <= tsq;
 }
 
-// Inlier counts of the homographies h < nh of the batch (S.H / S.hvalid ->
-// S.hcnt): warp w takes h = w, w + 8, ..., two per pass.  Ends with a barrier.
-static __device__ void h_count_batch(const RansacJob& J, RShared& S, int nh, int best) {
+// The f32 test of h_count_batch.  With M = max(Bx, By) + T Bw, where Bx = |h0| Qx + |h1|
+// Qy + |h2| bounds the terms of the numerator X over the set's matches (By, Bw alike) and
+// T the target coordinates, the f32 values of w and of U = X - tx w, V = Y - ty w are off
+// by at most 3.1 2^-24 Bw and 4.2 2^-24 M (H rounded, two fused steps each, one more for
+// U); the reference's f64 value of e is off from (U^2 + V^2) / w^2 by far less.  So with
+// G = thr (3.1 2^-24 Bw + 2e-9) + 6 2^-24 M (the 2e-9 keeps |w| >= 1e-9 certain) e <= thr^2
+// is certain for |(U, V)| <= thr |w| - G and excluded for |(U, V)| >= thr |w| + G, and
+// 2 thr |w| G <= k (thr w)^2 + G^2 / k, for any k, turns both into
+//   U^2 + V^2 <= w^2 lo.x + lo.y    and    U^2 + V^2 >= w^2 hi.x + hi.y.
+// In between, for values too large and for NaN the f64 test decides.
+static __device__ float4 h_band(const RShared& S, const double* H) {
+  const double Qx = __uint_as_float(S.coord_max[0]), Qy = __uint_as_float(S.coord_max[1]), T = __uint_as_float(S.coord_max[2]);
+  const double Bx = fabs(H[0]) * Qx + fabs(H[1]) * Qy + fabs(H[2]);
+  const double By = fabs(H[3]) * Qx + fabs(H[4]) * Qy + fabs(H[5]);
+  const double Bw = fabs(H[6]) * Qx + fabs(H[7]) * Qy + fabs(H[8]);
+  const double M = Bx + By + T * Bw, thr2 = S.tsq_d;  // Bx + By >= max(Bx, By), and holds a NaN
+  const double nan = __longlong_as_double(0x7ff8000000000000ll);
+  if (!(M < 1e15) || !(Bw < 1e15) || !(Qx < 1e15) || !(Qy < 1e15) || !(T < 1e15) || !(thr2 < 1e7))
+    return make_float4(-1.0f, 0.0f, (float)nan, 0.0f);
+  const double thr = sqrt(thr2);
+  const double G = 1.01 * (thr * (3.1 * 0x1p-24 * Bw + 2e-9) + 6.0 * 0x1p-24 * M);
+  const double k = fmin(fmax(G / thr, 0x1p-20), 0.5), s = 0x1p-20;  // s: the f32 roundings of the test itself
+  return make_float4((float)(thr2 * (1.0 - k) * (1.0 - s)), (float)(-G * G * (1.0 / k - 1.0) * (1.0 + s)),
+                     (float)(thr2 * (1.0 + k) * (1.0 + s)), (float)(G * G * (1.0 / k + 1.0) * (1.0 + s)));
+}
+
+// Inlier counts of the homographies h < nh of the batch (S.H / S.hband / S.hvalid ->
+// S.hcnt): warp w takes h = w, w + kRWarps, ..., two per pass over the matches.  The
+// staged matches (ns) are tested in packed f32, two per lane, the undecided ones in f64
+// (see h_band).  Ends with a barrier.
+// 88 hypotheses on 5650 matches: 606 k cycles in f64 (a division each, coordinates from
+// L2), 161 k like this.
+static __device__ void h_count_batch(const RansacJob& J, RShared& S, int nh, int best, int ns) {
+  extern __shared__ double jac[];
+  const float* xs = reinterpret_cast<const float*>(jac);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const double tsq = S.tsq_d;
-  for (int h = warp; h < nh; h += 2 * kRWarps) {
-    const int h2 = h + kRWarps;
-    const bool v1 = S.hvalid[h] != 0, v2 = h2 < nh && S.hvalid[h2] != 0;
-    int c1 = 0, c2 = 0;
-    double H1[9], H2[9];
+  constexpr int kPass = 2;
+  for (int h0 = warp; h0 < nh; h0 += kPass * kRWarps) {
+    bool v[kPass], go = false;
+    int c[kPass];
+    float2 H[kPass][9];
+    float4 band[kPass];
 #pragma unroll
-    for (int i = 0; i < 9; ++i) {
-      H1[i] = S.H[h][i];
-      H2[i] = v2 ? S.H[h2][i] : 0.0;
+    for (int u = 0; u < kPass; ++u) {
+      const int h = h0 + u * kRWarps;
+      v[u] = h < nh && S.hvalid[h] != 0;
+      c[u] = 0;
+      go |= v[u];
+#pragma unroll
+      for (int i = 0; i < 9; ++i) {
+        const float f = v[u] ? (float)S.H[h][i] : 0.0f;
+        H[u][i] = i < 6 ? make_float2(-f, -f) : make_float2(f, f);
+      }
+      band[u] = v[u] ? S.hband[h] : make_float4(-1.0f, -1.0f, 0.0f, 0.0f);  // an absent one: never in, always decided
     }
-    bool go = v1 || v2;
-    for (int i0 = 0; go && i0 < S.n; i0 += 32 * kCheck) {
+    auto exact = [&](int u, float4 p) {
+      double e;
+      return h_inlier(p, S.H[h0 + u * kRWarps], tsq, e);
+    };
+    auto reach = [&](int rest) {
+      bool any = false;
+#pragma unroll
+      for (int u = 0; u < kPass; ++u) any |= can_reach(v[u], c[u], rest, best);
+      return any;
+    };
+    for (int i0 = 0; go && i0 < ns; i0 += 32 * kCheck) {
+      const int i1 = min(i0 + 32 * kCheck, ns);
+      for (int i = i0 + 2 * lane; i < i1; i += 64) {
+        const float2 x = *reinterpret_cast<const float2*>(xs + i), y = *reinterpret_cast<const float2*>(xs + kStage + i);
+        const float2 z = *reinterpret_cast<const float2*>(xs + 2 * kStage + i), t = *reinterpret_cast<const float2*>(xs + 3 * kStage + i);
+        unsigned open = 0;  // bit 2 u + k: match k of the pair is undecided for u
+#pragma unroll
+        for (int u = 0; u < kPass; ++u) {
+          const float2 w = fma2(H[u][6], x, fma2(H[u][7], y, H[u][8]));
+          const float2 U = fma2(z, w, fma2(H[u][0], x, fma2(H[u][1], y, H[u][2])));  // minus the numerators
+          const float2 V = fma2(t, w, fma2(H[u][3], x, fma2(H[u][4], y, H[u][5])));
+          const float2 e = fma2(U, U, mul2(V, V)), w2 = mul2(w, w);
+          const float2 lo = fma2(w2, make_float2(band[u].x, band[u].x), make_float2(band[u].y, band[u].y));
+          const float2 hi = fma2(w2, make_float2(band[u].z, band[u].z), make_float2(band[u].w, band[u].w));
+          const bool in0 = e.x <= lo.x, in1 = e.y <= lo.y;
+          c[u] += in0 ? 1 : 0;
+          c[u] += in1 ? 1 : 0;
+          if (!in0 && !(e.x >= hi.x)) open |= 1u << (2 * u);
+          if (!in1 && !(e.y >= hi.y)) open |= 2u << (2 * u);
+        }
+        while (open) {
+          const int k = __ffs(open) - 1;
+          open &= open - 1;
+          const float4 p = k & 1 ? make_float4(x.y, y.y, z.y, t.y) : make_float4(x.x, y.x, z.x, t.x);
+          const int in = exact(k >> 1, p) ? 1 : 0;
+#pragma unroll
+          for (int u = 0; u < kPass; ++u) c[u] += k >> 1 == u ? in : 0;
+        }
+      }
+      go = reach(S.n - i1);
+    }
+    for (int i0 = ns; go && i0 < S.n; i0 += 32 * kCheck) {
       const int i1 = min(i0 + 32 * kCheck, S.n);
       for (int i = i0 + lane; i < i1; i += 32) {
         const float4 p = J.xy[i];
-        double e;
-        c1 += (v1 && h_inlier(p, H1, tsq, e)) ? 1 : 0;
-        c2 += (v2 && h_inlier(p, H2, tsq, e)) ? 1 : 0;
+#pragma unroll
+        for (int u = 0; u < kPass; ++u) c[u] += v[u] && exact(u, p) ? 1 : 0;
       }
-      go = can_reach(v1, c1, v2, c2, S.n - i1, best);
+      go = reach(S.n - i1);
     }
-    c1 = (int)__reduce_add_sync(0xffffffffu, (unsigned)c1);
-    c2 = (int)__reduce_add_sync(0xffffffffu, (unsigned)c2);
-    if (lane == 0) {
-      S.hcnt[h] = c1;
-      if (h2 < nh) S.hcnt[h2] = c2;
+#pragma unroll
+    for (int u = 0; u < kPass; ++u) {
+      const int h = h0 + u * kRWarps;
+      const int sum = (int)__reduce_add_sync(0xffffffffu, (unsigned)c[u]);
+      if (lane == 0 && h < nh) S.hcnt[h] = sum;
     }
   }
   __syncthreads();
 }
 
-static __device__ int h_count(const RansacJob& J, RShared& S, const double* H) {
+static __device__ int h_count(const RansacJob& J, RShared& S, const double* Hs) {
+  double H[9];
+  for (int i = 0; i < 9; ++i) H[i] = Hs[i];
   int c = 0;
   for (int i = threadIdx.x; i < S.n; i += kRThreads) {
     double e;
@@ -687,7 +872,9 @@ static __device__ int h_count(const RansacJob& J, RShared& S, const double* H) {
   return block_sum_int(c, S);
 }
 
-static __device__ double h_mass(const RansacJob& J, RShared& S, const double* H) {
+static __device__ double h_mass(const RansacJob& J, RShared& S, const double* Hs) {
+  double H[9];
+  for (int i = 0; i < 9; ++i) H[i] = Hs[i];
   double t = 0.0;
   for (int i = threadIdx.x; i < S.n && threadIdx.x < kMassThreads; i += kMassThreads) {
     double e;
@@ -707,7 +894,9 @@ static __device__ double h_err(const RansacJob& J, RShared& S, const double* H) 
   });
 }
 
-static __device__ int h_collect(const RansacJob& J, RShared& S, const double* H) {
+static __device__ int h_collect(const RansacJob& J, RShared& S, const double* Hs) {
+  double H[9];
+  for (int i = 0; i < 9; ++i) H[i] = Hs[i];
   int base = 0;
   for (int c0 = 0; c0 < S.n; c0 += kRThreads) {
     const int i = c0 + threadIdx.x;
@@ -732,16 +921,6 @@ static __device__ int h_collect(const RansacJob& J, RShared& S, const double* H)
   return base;
 }
 
-// Offset i * 9 + j of strict upper-triangle entry k (row-major, 36 entries).
-static __device__ __forceinline__ int strict_upper_offset(int k) {
-  int i = 0;
-  while (k >= 8 - i) {
-    k -= 8 - i;
-    ++i;
-  }
-  return i * 9 + i + 1 + k;
-}
-
 // (a, b), a <= b, of upper-triangle entry e (row-major, 45 entries).
 static __device__ __forceinline__ void upper_entry(int e, int& a, int& b) {
   a = 0;
@@ -754,65 +933,200 @@ static __device__ __forceinline__ void upper_entry(int e, int& a, int& b) {
 
 // smallest_eigenvector_9x9 (src/pipeline.rs:2276-2353), the cyclic Jacobi shared
 // by a quad of lanes (ql = 0..3, converged, qmask their lane mask).  A (81
-// doubles, shared memory, symmetric and complete) is diagonalised in place; V
-// (81 doubles) accumulates the eigenvectors.  Every lane computes each
-// rotation's parameters from the same values; lane ql updates rows ql, ql + 4,
-// ql + 8 (a rotation's row updates touch disjoint entries), so every value and
-// decision is the sequential solver's.  Returns the column of the smallest
-// diagonal entry (the first on ties), or -1 if that eigenvector is not finite.
-// A and V are complete and visible to the quad on return.
-static __device__ int quad_cyclic_jacobi(double* A, double* V, int ql, unsigned qmask) {
-  for (int r = ql; r < 9; r += 4)
+// doubles, shared memory, the upper triangle complete) is diagonalised in place; V
+// (81 doubles) receives the eigenvectors, a row each.  Returns the column of the
+// smallest diagonal entry (the first on ties), or -1 if that eigenvector is not
+// finite.  A's diagonal and V are complete and visible to the quad on return.
+// V must be A + 81 with A on a 16-byte boundary.
+//
+// A sweep's 36 rotations are a serial chain in the reference, and the chain of one
+// rotation's parameters (division, two square roots, two reciprocals in f64) is what
+// a fit takes its time for.  Two rotations without a common index do not read each
+// other's pivots, so rotation (p, r) runs at step p + r, up to four per step, one per
+// lane: 15 steps instead of 36.  Rounding does not commute, so every entry still sees
+// its updates in the reference's order:
+//   - a rotation (p, q) reaches column r > q when (p, r) is about to run (then every
+//     earlier rotation of index r has), so the lane of p first applies (p, p+1) ..
+//     (p, r-1) to column r, takes its pivot, and applies (p, r) to columns p+1 .. r-1;
+//   - what is left of a sweep touches rows whose own rotations are over (row i of A
+//     right of the diagonal, by rotations of indices above i) and the rows of V; these
+//     rows are independent of one another and are rotated once the sweep's parameters
+//     are known.
+// Every value and decision is the sequential solver's, bit by bit.  Bound by the latency
+// of a step (parameters 550 cycles).  Against the rotations one after the other, their
+// row updates shared by the lanes: 128 fits of a CTA 486 -> 293 k cycles, one fit (a
+// refit, 6 sweeps) 205 -> 141 k.
+// Volatile, or the compiler loads all of a sweep's parameters first, and spills.
+static __device__ __forceinline__ double2 rot_params(const double2* cs) {
+  double2 r;
+  asm volatile("ld.volatile.shared.v2.f64 {%0, %1}, [%2];" : "=d"(r.x), "=d"(r.y) : "r"((uint32_t)__cvta_generic_to_shared(cs)) : "memory");
+  return r;
+}
+static constexpr int kSkipHi = 0x40000000;  // c = 2: the rotation was skipped (a cosine is at most 1)
+static __device__ __noinline__ int quad_cyclic_jacobi(double* A, double* V, int ql, unsigned qmask) {
+  double2* CS = reinterpret_cast<double2*>(V + 1);  // (c, s) of the sweep's rotations, row-major
+  double va[9], vb[9];  // rows ql and ql + 4 of V; row 8 lives below A's diagonal
 #pragma unroll
-    for (int c = 0; c < 9; ++c) V[r * 9 + c] = r == c ? 1.0 : 0.0;
-  // this lane's 9 of the 36 upper-triangle entries (row-major entries ql, ql + 4, ...)
-  int off[9];
+  for (int c = 0; c < 9; ++c) {
+    va[c] = c == ql ? 1.0 : 0.0;
+    vb[c] = c == ql + 4 ? 1.0 : 0.0;
+  }
+  if (ql == 0) {
 #pragma unroll
-  for (int s = 0; s < 9; ++s) off[s] = strict_upper_offset(ql + 4 * s);
-  __syncwarp(qmask);
+    for (int c = 0; c < 8; ++c) A[72 + c] = 0.0;
+    A[63] = 1.0;
+  }
   for (int sweep = 0; sweep < 20; ++sweep) {
     double mx = 0.0;
 #pragma unroll
     for (int s = 0; s < 9; ++s) {
-      const double v = fabs(A[off[s]]);
+      const double v = fabs(A[kStrictUpper[ql + 4 * s]]);
       if (v > mx) mx = v;
     }
     mx = fmax(mx, __shfl_xor_sync(qmask, mx, 1));
     mx = fmax(mx, __shfl_xor_sync(qmask, mx, 2));
     if (mx < 1e-13) break;
-    for (int p = 0; p < 8; ++p)
-      for (int q = p + 1; q < 9; ++q) {
-        const double apq = A[p * 9 + q];
-        if (fabs(apq) < 1e-15) continue;
-        const double app = A[p * 9 + p], aqq = A[q * 9 + q];
-        const double tau = (aqq - app) / (2.0 * apq);
-        // __drcp_rn(x) is 1.0 / x: both are IEEE round-to-nearest, the reciprocal is the cheaper sequence
-        const double t = tau >= 0.0 ? __drcp_rn(tau + sqrt(1.0 + tau * tau)) : -__drcp_rn(-tau + sqrt(1.0 + tau * tau));
-        const double c = __drcp_rn(sqrt(1.0 + t * t));
-        const double s = t * c;
-        __syncwarp(qmask);  // every pivot read precedes the writes
-        if (ql == 0) {
-          A[p * 9 + p] = app - t * apq;
-          A[q * 9 + q] = aqq + t * apq;
-          A[p * 9 + q] = 0.0;
-          A[q * 9 + p] = 0.0;
-        }
-        for (int r = ql; r < 9; r += 4) {
-          if (r != p && r != q) {
-            const double arp = A[r * 9 + p], arq = A[r * 9 + q];
-            const double nrp = c * arp - s * arq, nrq = s * arp + c * arq;
-            A[r * 9 + p] = nrp;
-            A[p * 9 + r] = nrp;
-            A[r * 9 + q] = nrq;
-            A[q * 9 + r] = nrq;
-          }
-          const double vrp = V[r * 9 + p], vrq = V[r * 9 + q];
-          V[r * 9 + p] = c * vrp - s * vrq;
-          V[r * 9 + q] = s * vrp + c * vrq;
-        }
-        __syncwarp(qmask);
+    // the rotations' parameters and the entries they depend on
+#pragma unroll 1
+    for (int step = 1; step <= 15; ++step) {
+      int p = ql, r = step - ql;
+      if (r > 8) {
+        p += 4;
+        r -= 4;
       }
+      const int longest = step <= 8 ? step - 1 : 15 - step;  // of the step's columns, above the pivots
+      if (p < r && r <= 8) {
+        const int cnt = r - p - 1;
+        double* const row = A + p * 9 + p + 1;    // A[p][p + 1 + k] at [k]
+        double* const col = A + (p + 1) * 9 + r;  // A[p + 1 + k][r] at [9 k]
+        double2* const cs = CS + (p * (17 - p) >> 1);
+        double x = A[p * 9 + r];
+        double y[7];
+        // all seven slots at once or the first three, by the step's longest column; what
+        // lies beyond cnt is loaded (it is in the quad's memory) and not used
+        auto column = [&](auto first, auto last) {
+          constexpr int k0 = decltype(first)::value, k1 = decltype(last)::value;
+          double2 rot[k1];
+#pragma unroll
+          for (int k = k0; k < k1; ++k) {
+            rot[k] = cs[min(k, cnt)];
+            y[k] = col[9 * k];
+          }
+#pragma unroll
+          for (int k = k0; k < k1; ++k) {
+            const bool on = k < cnt && __double2hiint(rot[k].x) != kSkipHi;
+            const double nx = rot[k].x * x - rot[k].y * y[k], ny = rot[k].y * x + rot[k].x * y[k];
+            x = on ? nx : x;
+            y[k] = on ? ny : y[k];
+          }
+        };
+        if (longest > 0) column(Int<0>(), Int<3>());
+        if (longest > 3) column(Int<3>(), Int<7>());
+        const double apq = x;
+        const bool rotate = !(fabs(apq) < 1e-15);
+        double c = 2.0, s = 0.0;
+        if (rotate) {
+          const double app = A[p * 10], aqq = A[r * 10];
+          const double tau = (aqq - app) / (2.0 * apq);
+          // __drcp_rn(x) is 1.0 / x: both are IEEE round-to-nearest, the reciprocal is the cheaper sequence
+          const double m = __drcp_rn(fabs(tau) + sqrt(1.0 + tau * tau)), t = tau >= 0.0 ? m : -m;
+          c = __drcp_rn(sqrt(1.0 + t * t));
+          s = t * c;
+          A[p * 10] = app - t * apq;
+          A[r * 10] = aqq + t * apq;
+        }
+        cs[cnt] = make_double2(c, s);
+        row[cnt] = rotate ? 0.0 : apq;
+        auto rest = [&](auto first, auto last) {
+          constexpr int k0 = decltype(first)::value, k1 = decltype(last)::value;
+          double a[k1];
+#pragma unroll
+          for (int k = k0; k < k1; ++k) a[k] = row[k];
+#pragma unroll
+          for (int k = k0; k < k1; ++k) {
+            const double na = c * a[k] - s * y[k], ny = s * a[k] + c * y[k];
+            if (k < cnt && rotate) row[k] = na;
+            if (k < cnt) col[9 * k] = rotate ? ny : y[k];
+          }
+        };
+        if (longest > 0) rest(Int<0>(), Int<3>());
+        if (longest > 3) rest(Int<3>(), Int<7>());
+      }
+      __syncwarp(qmask);
+    }
+    // V's rows ql and ql + 4
+#pragma unroll
+    for (int p = 0; p < 8; ++p) {
+#pragma unroll
+      for (int q = p + 1; q < 9; ++q) {
+        const double2 rot = rot_params(CS + p * (17 - p) / 2 + q - p - 1);
+        if (__double2hiint(rot.x) != kSkipHi) {
+          const double ap = va[p], aq = va[q], bp = vb[p], bq = vb[q];
+          va[p] = rot.x * ap - rot.y * aq;
+          va[q] = rot.y * ap + rot.x * aq;
+          vb[p] = rot.x * bp - rot.y * bq;
+          vb[q] = rot.y * bp + rot.x * bq;
+        }
+      }
+    }
+    {  // row 8 of V (lane 0), rows 0, 1, 2 of A right of the diagonal
+      double* const base = ql == 0 ? A + 72 : A + (ql - 1) * 9;
+      double* const last = ql == 0 ? A + 63 : base + 8;
+      double x[9];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) x[c] = base[c];
+      x[8] = *last;
+#pragma unroll
+      for (int p = 0; p < 8; ++p) {
+#pragma unroll
+        for (int q = p + 1; q < 9; ++q) {
+          const double2 rot = rot_params(CS + p * (17 - p) / 2 + q - p - 1);
+          if (p >= ql && __double2hiint(rot.x) != kSkipHi) {
+            const double xp = x[p], xq = x[q];
+            x[p] = rot.x * xp - rot.y * xq;
+            x[q] = rot.y * xp + rot.x * xq;
+          }
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < 8; ++c)
+        if (c >= ql) base[c] = x[c];
+      *last = x[8];
+    }
+    {  // rows 3 .. 6 of A
+      double* const base = A + (3 + ql) * 9;
+      double x[9];
+#pragma unroll
+      for (int c = 4; c < 9; ++c) x[c] = base[c];
+#pragma unroll
+      for (int p = 4; p < 8; ++p)
+#pragma unroll
+        for (int q = p + 1; q < 9; ++q) {
+          const double2 rot = rot_params(CS + p * (17 - p) / 2 + q - p - 1);
+          if (p > 3 + ql && __double2hiint(rot.x) != kSkipHi) {
+            const double xp = x[p], xq = x[q];
+            x[p] = rot.x * xp - rot.y * xq;
+            x[q] = rot.y * xp + rot.x * xq;
+          }
+        }
+#pragma unroll
+      for (int c = 4; c < 9; ++c)
+        if (c > 3 + ql) base[c] = x[c];
+    }
+    __syncwarp(qmask);
   }
+  __syncwarp(qmask);  // V takes the place of the parameters
+#pragma unroll
+  for (int c = 0; c < 9; ++c) {
+    V[ql * 9 + c] = va[c];
+    V[(ql + 4) * 9 + c] = vb[c];
+  }
+  if (ql == 0) {
+#pragma unroll
+    for (int c = 0; c < 8; ++c) V[72 + c] = A[72 + c];
+    V[80] = A[63];
+  }
+  __syncwarp(qmask);
   int mi = 0;
   double me = A[0];
   for (int i = 1; i < 9; ++i)
@@ -928,8 +1242,8 @@ static __device__ bool quad_fit4(const float4* __restrict__ xy, const int* idx, 
 }
 
 // fit_homography_dlt_f64 over J.list[0..k) (k >= 4), whole CTA; jac holds one
-// free A / V pair.  Result in H (every thread); false if the fit fails.
-static __device__ bool fit_dlt_list(const RansacJob& J, RShared& S, double* jac, int k, double* H) {
+// free A / V pair.  Result in S.dres[0 .. 8]; false if the fit fails.
+static __device__ bool fit_dlt_list(const RansacJob& J, RShared& S, double* jac, int k) {
   const double inv_n = 1.0 / (double)k;
   // The inliers' points (list order) staged in shared memory a chunk at a time;
   // every sum below stays sequential in list order, its terms read at
@@ -1051,7 +1365,6 @@ static __device__ bool fit_dlt_list(const RansacJob& J, RShared& S, double* jac,
   }
   __syncthreads();
   const bool ok = S.flag != 0;
-  for (int i = 0; i < 9; ++i) H[i] = S.dres[i];
   __syncthreads();
   return ok;
 }
@@ -1071,44 +1384,56 @@ static __device__ bool degenerate4(const double (&p)[4][2]) {
   return false;
 }
 
-// local_optimize_homography (src/pipeline.rs:2605-2631); updates H / count /
-// err in place (err valid when err_known; computed only for a tie).
+// local_optimize_homography (src/pipeline.rs:2605-2631); updates H (shared memory) /
+// count / err in place (err valid when err_known; computed only for a tie).
 static __device__ void local_optimize(const RansacJob& J, RShared& S, double* jac, double* H, int& count, double& err,
                                bool& err_known) {
   for (int round = 0; round < 2; ++round) {
     const int k = h_collect(J, S, H);
     if (k < 4) break;
-    double R[9];
-    if (!fit_dlt_list(J, S, jac, k, R)) break;
-    const int rc = h_count(J, S, R);
+    if (!fit_dlt_list(J, S, jac, k)) break;
+    const int rc = h_count(J, S, S.dres);
     if (rc < count) break;
     if (rc == count) {
       if (!err_known) {
         err = h_err(J, S, H);
         err_known = true;
       }
-      const double re = h_err(J, S, R);
+      const double re = h_err(J, S, S.dres);
       if (!(re < err)) break;
       err = re;
     } else {
       err_known = false;
     }
-    for (int i = 0; i < 9; ++i) H[i] = R[i];
+    if (threadIdx.x < 9) H[threadIdx.x] = S.dres[threadIdx.x];
+    __syncthreads();
     count = rc;
   }
 }
 
-static __device__ void run(const RansacJob& J, RShared& S) {
+static __device__ void run(const RansacJob& J, RShared& S, float one) {
   extern __shared__ double jac[];
   const int n = J.n;
   if (threadIdx.x == 0) S.n = n;
+  if (threadIdx.x < 3) S.coord_max[threadIdx.x] = 0;
+  __syncthreads();
+  unsigned mx[3] = {0, 0, 0};  // as bits: a NaN exceeds every number
   for (int i = threadIdx.x; i < n; i += kRThreads) {
     J.mask[i] = 0;
     const psift_match& m = J.m[i];
-    J.xy[i] = make_float4(m.query_x, m.query_y, m.target_x, m.target_y);
+    const float4 p = make_float4(m.query_x, m.query_y, m.target_x, m.target_y);
+    J.xy[i] = p;
+    mx[0] = max(mx[0], __float_as_uint(fabsf(p.x)));
+    mx[1] = max(mx[1], __float_as_uint(fabsf(p.y)));
+    mx[2] = max(mx[2], max(__float_as_uint(fabsf(p.z)), __float_as_uint(fabsf(p.w))));
+  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const unsigned w = __reduce_max_sync(0xffffffffu, mx[k]);
+    if ((threadIdx.x & 31) == 0) atomicMax(&S.coord_max[k], w);
   }
   __syncthreads();
-  similarity_ransac(J, S, jac, J.sim_seed, J.thr);
+  similarity_ransac(J, S, jac, J.sim_seed, J.thr, one);
   if (!J.homography) {
     const int k = S.sim_count;
     for (int j = threadIdx.x; j < k; j += kRThreads) J.mask[J.list[j]] = 1;
@@ -1125,13 +1450,14 @@ static __device__ void run(const RansacJob& J, RShared& S) {
   __syncthreads();
   // The incumbent, held identically by every thread.
   bool has_bh = S.has_sim != 0;
-  double BH[9];
-  {
+  double* const BH = S.BH;
+  if (threadIdx.x == 0) {
     const double a = S.sim_model[0], b = S.sim_model[1];
     BH[0] = a, BH[1] = -b, BH[2] = S.sim_model[2];
     BH[3] = b, BH[4] = a, BH[5] = S.sim_model[3];
     BH[6] = 0.0, BH[7] = 0.0, BH[8] = 1.0;
   }
+  __syncthreads();
   int best_count = 0;
   double best_err = __longlong_as_double(0x7ff0000000000000ll);
   bool err_known = true;
@@ -1179,32 +1505,57 @@ static __device__ void run(const RansacJob& J, RShared& S) {
       __syncthreads();
       if (threadIdx.x == 0) {
         S.draws_ready = need < draw_cap ? need : draw_cap;
-        int p = S.draw_ptr;
-        for (int h = 0; h < nh; ++h) {
-          // distinct draws in order, held in registers (q0 first)
-          int chosen = 0, attempts = 0;
-          int q0 = 0, q1 = 0, q2 = 0, q3 = 0;
-          while (chosen < 4 && attempts < 16) {
-            ++attempts;
-            const int c = S.draws_s[(p++) % (2 * kDrawChunk)];
-            const bool dup = (chosen > 0 && q0 == c) || (chosen > 1 && q1 == c) || (chosen > 2 && q2 == c);
-            if (!dup) {
-              if (chosen == 0) q0 = c;
-              else if (chosen == 1) q1 = c;
-              else if (chosen == 2) q2 = c;
-              else q3 = c;
-              ++chosen;
-            }
-          }
-          S.quad[h][0] = q0;
-          S.quad[h][1] = q1;
-          S.quad[h][2] = q2;
-          S.quad[h][3] = q3;
-          S.hvalid[h] = chosen == 4 ? 1 : 0;
-        }
-        S.draw_ptr = p;
+        S.dup = kBatch;
       }
       __syncthreads();
+      // Almost every sample's first 4 draws are distinct: sample done + k then uses draws
+      // p + 4 k .. p + 4 k + 3 up to the first one with a repeat, which thread 0 takes as
+      // the reference does; the rest follow in the next turn.
+      for (int done = 0; done < nh;) {
+        const int p = S.draw_ptr, h = done + (int)threadIdx.x;
+        if (h < nh) {
+          int q[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) q[k] = S.draws_s[(p + 4 * (int)threadIdx.x + k) % (2 * kDrawChunk)];
+          const bool dup = q[0] == q[1] || q[0] == q[2] || q[0] == q[3] || q[1] == q[2] || q[1] == q[3] || q[2] == q[3];
+          if (dup) atomicMin(&S.dup, h);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) S.quad[h][k] = q[k];
+          S.hvalid[h] = 1;
+        }
+        __syncthreads();
+        const int first = min(S.dup, nh);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+          int p0 = p + 4 * (first - done);
+          if (first < nh) {
+            // distinct draws in order, held in registers (q0 first)
+            int chosen = 0, attempts = 0;
+            int q0 = 0, q1 = 0, q2 = 0, q3 = 0;
+            while (chosen < 4 && attempts < 16) {
+              ++attempts;
+              const int c = S.draws_s[(p0++) % (2 * kDrawChunk)];
+              const bool dup = (chosen > 0 && q0 == c) || (chosen > 1 && q1 == c) || (chosen > 2 && q2 == c);
+              if (!dup) {
+                if (chosen == 0) q0 = c;
+                else if (chosen == 1) q1 = c;
+                else if (chosen == 2) q2 = c;
+                else q3 = c;
+                ++chosen;
+              }
+            }
+            S.quad[first][0] = q0;
+            S.quad[first][1] = q1;
+            S.quad[first][2] = q2;
+            S.quad[first][3] = q3;
+            S.hvalid[first] = chosen == 4 ? 1 : 0;
+            S.dup = kBatch;
+          }
+          S.draw_ptr = p0;
+        }
+        __syncthreads();
+        done = min(first + 1, nh);
+      }
     }
     // fits: a quad of lanes per hypothesis
     {
@@ -1225,15 +1576,18 @@ static __device__ void run(const RansacJob& J, RShared& S) {
         } else {
           double Hh[9];
           valid = quad_fit4(J.xy, S.quad[h], jac + h * 162, jac + h * 162 + 81, ql, qmask, Hh);
-          if (valid && ql == 0)
+          if (valid && ql == 0) {
             for (int i = 0; i < 9; ++i) S.H[h][i] = Hh[i];
+            S.hband[h] = h_band(S, Hh);
+          }
         }
       }
       __syncwarp();  // every lane of the quad has read S.hvalid[h]
       if (ql == 0) S.hvalid[h] = valid ? 1 : 0;
     }
     __syncthreads();
-    h_count_batch(J, S, nh, best_count);
+    const int ns = stage_coords(J, S);
+    h_count_batch(J, S, nh, best_count, ns);
     // replay in order
     for (int h = 0; h < nh; ++h) {
       const int it = base + h;
@@ -1256,13 +1610,15 @@ static __device__ void run(const RansacJob& J, RShared& S) {
         e_known = true;
         if (!(e < best_err)) continue;
       }
-      double Hc[9];
-      for (int i = 0; i < 9; ++i) Hc[i] = S.H[h][i];
-      local_optimize(J, S, jac, Hc, c, e, e_known);
+      if (threadIdx.x < 9) S.Hc[threadIdx.x] = S.H[h][threadIdx.x];
+      __syncthreads();
+      local_optimize(J, S, jac, S.Hc, c, e, e_known);
       best_count = c;
       best_err = e;
       err_known = e_known;
-      for (int i = 0; i < 9; ++i) BH[i] = Hc[i];
+      __syncthreads();
+      if (threadIdx.x < 9) BH[threadIdx.x] = S.Hc[threadIdx.x];
+      __syncthreads();
       has_bh = true;
       max_iters = guided ? adaptive_iters_w(h_mass(J, S, BH) / wtot, 4, 64, 2000)
                          : adaptive_iters(best_count, n, 4, 64, 2000);
@@ -1288,9 +1644,9 @@ static __device__ void run(const RansacJob& J, RShared& S) {
 };
 
 template <int THREADS>
-__global__ void __launch_bounds__(THREADS, 512 / THREADS) ransac_kernel(const RansacJob* __restrict__ jobs) {
+__global__ void __launch_bounds__(THREADS, 512 / THREADS) ransac_kernel(const RansacJob* __restrict__ jobs, float one) {
   __shared__ typename RansacCta<THREADS>::RShared S;
-  RansacCta<THREADS>::run(jobs[blockIdx.x], S);
+  RansacCta<THREADS>::run(jobs[blockIdx.x], S, one);
 }
 
 template <int THREADS>
@@ -1298,7 +1654,7 @@ static cudaError_t launch_ransac_t(const RansacJob* jobs, int n_jobs, cudaStream
   constexpr size_t smem = RansacCta<THREADS>::kJacSmem;
   cudaError_t e = ensure_smem_attr((const void*)ransac_kernel<THREADS>, smem);
   if (e != cudaSuccess) return e;
-  ransac_kernel<THREADS><<<n_jobs, THREADS, smem, st>>>(jobs);
+  ransac_kernel<THREADS><<<n_jobs, THREADS, smem, st>>>(jobs, 1.0f);
   return cudaGetLastError();
 }
 
