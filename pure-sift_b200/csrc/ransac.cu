@@ -70,12 +70,11 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) {
 static __constant__ uint8_t kStrictUpper[36] = {1,  2,  3,  4,  5,  6,  7,  8,  11, 12, 13, 14, 15, 16, 17, 21, 22, 23,
                                                 24, 25, 26, 31, 32, 33, 34, 35, 41, 42, 43, 44, 51, 52, 53, 61, 62, 71};
 
-// A CTA's threads, by the number of match sets of a launch.  The serial parts (replay,
-// sequential sums, the Jacobi of a refit) leave most of a CTA idle, so many sets
-// share the SMs best as four CTAs of 128 threads each (128 registers, ~51 KB of
-// shared memory).  Up to one set per SM a CTA may use the whole SM: 512 threads fit
-// and count four times the hypotheses of a batch in about the time of 32, which is
-// what a set with many outliers spends its time on.
+// A CTA's threads, by the number of match sets of a launch.  512 threads fit and count
+// the most hypotheses at a time, which is what a set with many outliers spends its time
+// on, and take a whole SM; the serial parts (replay, sequential sums, the Jacobi of a
+// refit) leave most of them idle, so once there are several sets per SM two CTAs of
+// 256 threads side by side (128 registers, ~100 KB of shared memory) get more done.
 template <int THREADS>
 struct RansacCta {
 static constexpr int kRThreads = THREADS;
@@ -1658,15 +1657,13 @@ static cudaError_t launch_ransac_t(const RansacJob* jobs, int n_jobs, cudaStream
   return cudaGetLastError();
 }
 
-// 128 sets of 2000 to 8000 matches (outliers 10 to 70 %): 6.9 ms with 512 threads per
-// set, 19.4 with 128; one set of 470 matches 0.65 against 0.92 ms.  Above one set per
-// SM the 512-thread CTAs would run in waves; up to two, 256 threads still fit side by
-// side; beyond, four 128-thread CTAs per SM overlap the most sets (1024 sets: 26 ms).
+// Sets of 2000 to 7640 matches, outliers 10 to 70 %, milliseconds with 512 / 256 threads
+// per set: 128 sets 3.5 / 5.3, 296 5.5 / 6.0, 444 6.9 / 7.1, 500 7.6 / 7.5, 740 10.5 /
+// 9.5, 1024 13.3 / 11.5 (128 threads, four CTAs per SM: 12.0 to 16.7); one set of 470
+// 0.57 / 0.64.
 cudaError_t launch_ransac(const RansacJob* jobs, int n_jobs, int num_sms, cudaStream_t st) {
   if (n_jobs <= 0) return cudaSuccess;
-  if (n_jobs <= num_sms) return launch_ransac_t<512>(jobs, n_jobs, st);
-  if (n_jobs <= 2 * num_sms) return launch_ransac_t<256>(jobs, n_jobs, st);
-  return launch_ransac_t<128>(jobs, n_jobs, st);
+  return n_jobs <= 3 * num_sms ? launch_ransac_t<512>(jobs, n_jobs, st) : launch_ransac_t<256>(jobs, n_jobs, st);
 }
 
 }  // namespace psift

@@ -1,4 +1,4 @@
-"""RANSAC CTAs of 512, 256 and 128 threads (chosen by the number of sets of a launch): a
+"""RANSAC CTAs of 512 and 256 threads (chosen by the number of sets of a launch): a
 set's result does not depend on the launch it is part of."""
 import numpy as np
 import pytest
@@ -25,7 +25,7 @@ def test_result_does_not_depend_on_the_number_of_sets(homography, guided):
     run = lambda reps: psift.ransac_batch([m for m, _ in sets] * reps, homography=homography,  # noqa: E731
                                           weights=[w for _, w in sets] * reps if guided else None, ctx=ctx)
     one = run(1)  # 24 sets: 512 threads each
-    for reps in (10, 13):  # 240: 256 threads; 312: 128 threads
+    for reps in (10, 20):  # 240: 512 threads; 480: 256 threads
         many = run(reps)
         for i, (mask, model, iters) in enumerate(many):
             m1, h1, it1 = one[i % 24]
