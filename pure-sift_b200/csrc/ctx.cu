@@ -29,6 +29,7 @@ psift_status arena_reserve(psift_ctx* ctx, size_t bytes) {
     cudaError_t e = cudaMalloc(&ctx->arena.base, bytes);
     if (e != cudaSuccess) {
       ctx->arena.base = nullptr;
+      (void)cudaGetLastError();  // not a later launch's error: the caller may go on with less
       return cuda_error(ctx, e, "cudaMalloc(workspace)");
     }
     ctx->arena.capacity = bytes;

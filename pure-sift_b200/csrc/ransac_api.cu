@@ -111,13 +111,14 @@ psift_status estimate_host(psift_ctx* ctx, const psift_match* m, uint32_t n, con
 
 // The similarity and the homography estimations of the same match lists (both callers
 // want both): one launch when every job gets an SM of its own, so that the two run side
-// by side instead of one after the other.
+// by side instead of one after the other (and the scratch of both fits).
 psift_status ransac_both_dev(psift_ctx* ctx, const std::vector<psift_ransac_job>& sim,
                              const std::vector<psift_ransac_job>& hom, const psift_ransac_options& opt) {
   if (sim.size() + hom.size() <= (size_t)ctx->num_sms) {
     std::vector<psift_ransac_job> all(sim);
     all.insert(all.end(), hom.begin(), hom.end());
-    return run_batch(ctx, all.data(), (int)all.size(), opt, (int)sim.size());
+    const psift_status st = run_batch(ctx, all.data(), (int)all.size(), opt, (int)sim.size());
+    if (st != PSIFT_ERR_OUT_OF_MEMORY) return st;
   }
   const psift_status st = run_batch(ctx, sim.data(), (int)sim.size(), opt, (int)sim.size());
   return st != PSIFT_OK ? st : run_batch(ctx, hom.data(), (int)hom.size(), opt, 0);

@@ -61,3 +61,31 @@ def test_candidates_that_overflow():
     for k in (1, 40, 64):
         _check(q, c, k, ctx)
     ctx.close()
+
+
+def test_query_blocks_of_a_full_device():
+    # 8192 queries need 68 MB of scratch; with 32 MB left they are taken 1024 at a time
+    import ctypes as C
+
+    import torch
+    rng = np.random.default_rng(5)
+    c = rng.integers(0, 2 ** 64, (5000, 2), dtype=np.uint64)
+    q = rng.integers(0, 2 ** 64, (8192, 2), dtype=np.uint64)
+    _check(q[:4], c, 8)  # the kernels are loaded
+    ctx = psift.Context(0)
+    dq, dc = (torch.from_numpy(a.view(np.int64)).cuda() for a in (q, c))
+    idx, dist = (torch.zeros((len(q), 8), dtype=torch.int32, device="cuda") for _ in range(2))
+    free = torch.cuda.mem_get_info()[0]
+    fill = torch.empty(free - (32 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        ctx.check(ctx.lib.psift_hamming_topk_dev(ctx.handle, C.c_void_p(dq.data_ptr()), len(q),
+                                                 C.c_void_p(dc.data_ptr()), len(c), 8, C.c_void_p(idx.data_ptr()),
+                                                 C.c_void_p(dist.data_ptr())))
+        ctx.synchronize()
+    finally:
+        del fill
+        torch.cuda.empty_cache()
+    ri, rd = O.hamming_topk(q, c, 8)
+    np.testing.assert_array_equal(idx.cpu().numpy().view(np.uint32), ri)
+    np.testing.assert_array_equal(dist.cpu().numpy().view(np.uint32), rd)
+    ctx.close()
