@@ -187,6 +187,14 @@ psift_status pinned_reserve(psift_ctx* ctx, size_t bytes) {
   return PSIFT_OK;
 }
 
+// The context's streams and events, as far as they exist.
+static void destroy_streams(psift_ctx* ctx) {
+  for (cudaEvent_t e : {ctx->ev_fork, ctx->ev_join, ctx->ev_tail[0], ctx->ev_tail[1]})
+    if (e) cudaEventDestroy(e);
+  for (cudaStream_t s : {ctx->tail[0], ctx->tail[1], ctx->stream2, ctx->stream})
+    if (s) cudaStreamDestroy(s);
+}
+
 }  // namespace psift
 
 extern "C" {
@@ -208,22 +216,18 @@ psift_status psift_ctx_create(int device, psift_ctx** out) {
     delete ctx;
     return PSIFT_ERR_CUDA;
   }
-  if (cudaStreamCreateWithFlags(&ctx->stream2, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
-      cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming) != cudaSuccess) {
-    if (ctx->stream2) cudaStreamDestroy(ctx->stream2);
-    if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
-    cudaStreamDestroy(ctx->stream);
+  bool ok = cudaStreamCreateWithFlags(&ctx->stream2, cudaStreamNonBlocking) == cudaSuccess &&
+            cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming) == cudaSuccess &&
+            cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming) == cudaSuccess;
+  for (int c = 0; c < 2; ++c)
+    ok = ok && cudaStreamCreateWithFlags(&ctx->tail[c], cudaStreamNonBlocking) == cudaSuccess &&
+         cudaEventCreateWithFlags(&ctx->ev_tail[c], cudaEventDisableTiming) == cudaSuccess;
+  const bool mem = ok && cudaMalloc(&ctx->d_error, 64) == cudaSuccess && cudaMemset(ctx->d_error, 0, 64) == cudaSuccess;
+  if (!mem) {
+    if (ctx->d_error) cudaFree(ctx->d_error);
+    psift::destroy_streams(ctx);
     delete ctx;
-    return PSIFT_ERR_CUDA;
-  }
-  if (cudaMalloc(&ctx->d_error, 64) != cudaSuccess || cudaMemset(ctx->d_error, 0, 64) != cudaSuccess) {
-    cudaStreamDestroy(ctx->stream2);
-    cudaEventDestroy(ctx->ev_fork);
-    cudaEventDestroy(ctx->ev_join);
-    cudaStreamDestroy(ctx->stream);
-    delete ctx;
-    return PSIFT_ERR_OUT_OF_MEMORY;
+    return ok ? PSIFT_ERR_OUT_OF_MEMORY : PSIFT_ERR_CUDA;
   }
   *out = ctx;
   return PSIFT_OK;
@@ -234,6 +238,7 @@ psift_status psift_ctx_destroy(psift_ctx* ctx) {
   cudaSetDevice(ctx->device);
   cudaStreamSynchronize(ctx->stream);
   cudaStreamSynchronize(ctx->stream2);
+  for (cudaStream_t t : ctx->tail) cudaStreamSynchronize(t);
   if (ctx->arena.base) cudaFree(ctx->arena.base);
   if (ctx->io.base) cudaFree(ctx->io.base);
   if (ctx->stitch.base) cudaFree(ctx->stitch.base);
@@ -248,10 +253,7 @@ psift_status psift_ctx_destroy(psift_ctx* ctx) {
   for (cudaEvent_t e : ctx->timer.pool) cudaEventDestroy(e);
   for (auto& g : ctx->graphs)
     if (g.second.exec) cudaGraphExecDestroy(g.second.exec);
-  cudaEventDestroy(ctx->ev_fork);
-  cudaEventDestroy(ctx->ev_join);
-  cudaStreamDestroy(ctx->stream2);
-  cudaStreamDestroy(ctx->stream);
+  psift::destroy_streams(ctx);
   delete ctx;
   return PSIFT_OK;
 }

@@ -289,10 +289,23 @@ cudaError_t launch_level(const DetectJob& job, const SigmaSchedule& sc, int o, i
                      job.blur_fused, &tm, job.plans.data(), err);
 }
 
+// Octave-0 pixels of a launch up to which an octave's last levels run beside the next
+// octave.  Microseconds on one stream / beside (upsampled, 4 octaves): one 320 x 240 image
+// on the host 269 / 229, 640 x 480 346 / 305, 1920 x 1080 (8.3 M pixels) 726 / 678; device
+// batches, halves of two 640 x 480 381 / 332, of one 1920 x 1080 654 / 627.  Where a launch
+// fills the chip it gives nothing: halves of four 1920 x 1080 (33 M) 1900 / 1896, of six
+// images up to 23 M 2772 / 2794.
+constexpr long long kTailMaxPixels = 12000000;
+
 // Queue every stage of the path for the batch (no host synchronisation).
 // stop_after_keypoints: end after extrema_emit (Sift::detect_keypoints).
+// tail (with its event): octave o + 1 needs octave o's level S only, so levels S + 1 and
+// S + 2 and the extrema of every octave but the last go to this side stream and run
+// beside the next octave, as long as the launches are too small to fill the chip
+// (kTailMaxPixels).
 psift_status launch_detect(psift_ctx* ctx, DetectJob& job, const psift_sift_config& cfg, bool stop_after_keypoints,
-                           cudaStream_t stream = nullptr, bool plans_uploaded = false) {
+                           cudaStream_t stream = nullptr, bool plans_uploaded = false, cudaStream_t tail = nullptr,
+                           cudaEvent_t ev_tail = nullptr) {
   cudaStream_t st = stream ? stream : ctx->stream;
   const int n = job.n;
   const int S = (int)cfg.scales;
@@ -341,21 +354,34 @@ psift_status launch_detect(psift_ctx* ctx, DetectJob& job, const psift_sift_conf
     const float mult = base_mult * (float)(1ull << o);
     for (int s = 0; s <= S && s < 11; ++s) xp.eff_scale[o][s] = kBaseSigma * mult * powi_f(sc.k, s);
   }
+  long long pixels = 0;
+  for (int i = 0; i < n; ++i)
+    if (job.n_oct[i] > 0) pixels += (long long)job.oct[(size_t)i * kMaxOctaves].h * job.oct[(size_t)i * kMaxOctaves].w;
+  if (pixels > kTailMaxPixels || max_oct < 2) tail = nullptr;
   for (int o = 0; o < max_oct; ++o) {
     int mh, mw;
     max_dims(o, mh, mw);
+    const cudaStream_t last = tail && o + 1 < max_oct ? tail : st;  // stream of the octave's last part
     {
       StageScope sc_pyr(ctx, STAGE_PYRAMID, st);
       for (int s = 1; s <= S + 2; ++s) {
-        cudaError_t e = launch_level(job, sc, o, s, S, mh, mw, st, ctx->d_error);
+        cudaError_t e = launch_level(job, sc, o, s, S, mh, mw, s <= S ? st : last, ctx->d_error);
         ctx->launches++;
         if (e != cudaSuccess) return cuda_error(ctx, e, "blur(level)");
+        if (s == S && last != st) {
+          PSIFT_CUDA_TRY(ctx, cudaEventRecord(ev_tail, st));
+          PSIFT_CUDA_TRY(ctx, cudaStreamWaitEvent(tail, ev_tail, 0));
+        }
       }
     }
     StageScope sc_x(ctx, STAGE_EXTREMA, st);
-    cudaError_t e = launch_extrema_mark(job.d_plans, n, o, mh, mw, xp, st);
+    cudaError_t e = launch_extrema_mark(job.d_plans, n, o, mh, mw, xp, last);
     ctx->launches++;
     if (e != cudaSuccess) return cuda_error(ctx, e, "extrema_mark");
+  }
+  if (tail) {
+    PSIFT_CUDA_TRY(ctx, cudaEventRecord(ev_tail, tail));
+    PSIFT_CUDA_TRY(ctx, cudaStreamWaitEvent(st, ev_tail, 0));
   }
   cudaError_t e;
   {
@@ -456,7 +482,7 @@ bool is_host_pinned(const void* p) {
 
 psift_status launch_detect_split(psift_ctx* ctx, DetectJob& job, const psift_sift_config& cfg) {
   const int n = job.n;
-  if (n < 2) return launch_detect(ctx, job, cfg, false, nullptr, true);
+  if (n < 2) return launch_detect(ctx, job, cfg, false, nullptr, true, ctx->tail[0], ctx->ev_tail[0]);
   PSIFT_CUDA_TRY(ctx, cudaEventRecord(ctx->ev_fork, ctx->stream));
   PSIFT_CUDA_TRY(ctx, cudaStreamWaitEvent(ctx->stream2, ctx->ev_fork, 0));
   const int split = (n + 1) / 2;
@@ -473,7 +499,7 @@ psift_status launch_detect_split(psift_ctx* ctx, DetectJob& job, const psift_sif
     v.sel_cap = job.sel_cap;
     std::memcpy(v.blur_variant, job.blur_variant, sizeof v.blur_variant);  // the context's tuning
     v.blur_fused = job.blur_fused;
-    psift_status st = launch_detect(ctx, v, cfg, false, streams[c], true);
+    psift_status st = launch_detect(ctx, v, cfg, false, streams[c], true, ctx->tail[c], ctx->ev_tail[c]);
     if (st != PSIFT_OK) return st;
   }
   PSIFT_CUDA_TRY(ctx, cudaEventRecord(ctx->ev_join, ctx->stream2));

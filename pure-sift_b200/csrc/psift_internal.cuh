@@ -66,6 +66,10 @@ struct psift_ctx {
   // that fork it from and join it back to `stream`.
   cudaStream_t stream2 = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  // Side streams of the detection (one per half of a batch): the levels and extrema of
+  // an octave that the next octave does not wait for (launch_detect).
+  cudaStream_t tail[2] = {nullptr, nullptr};
+  cudaEvent_t ev_tail[2] = {nullptr, nullptr};
   std::string last_error;
   uint64_t launches = 0;
   psift::DeviceArena arena;   // per-call workspace
