@@ -32,8 +32,8 @@ cudaError_t launch_extrema_mark(const ImagePlan* plans, int n, int octave, int m
 cudaError_t launch_dog_plane(const float* lower, const float* upper, long long pitch, int h, int w, float* out,
                              cudaStream_t st);
 cudaError_t launch_row_scan(const ImagePlan* plans, int n, uint32_t kp_cap, uint32_t* err, cudaStream_t st);
-cudaError_t launch_extrema_emit(const ImagePlan* plans, int n, int octave, int max_h, const ExtremaParams& prm,
-                                uint32_t kp_cap, cudaStream_t st);
+cudaError_t launch_extrema_emit(const ImagePlan* plans, int n, int max_rows, const ExtremaParams& prm, uint32_t kp_cap,
+                                cudaStream_t st);
 cudaError_t launch_select_topk(const ImagePlan* plans, int n, uint32_t kp_cap, uint32_t max_features, uint32_t* err,
                                cudaStream_t st);
 cudaError_t launch_orientation(const ImagePlan* plans, int n, uint32_t sel_cap, const DescribeParams& prm,
@@ -389,13 +389,11 @@ psift_status launch_detect(psift_ctx* ctx, DetectJob& job, const psift_sift_conf
   e = launch_row_scan(job.d_plans, n, job.kp_cap, ctx->d_error, st);
   ctx->launches++;
   if (e != cudaSuccess) return cuda_error(ctx, e, "row_scan");
-  for (int o = 0; o < max_oct; ++o) {
-    int mh, mw;
-    max_dims(o, mh, mw);
-    e = launch_extrema_emit(job.d_plans, n, o, mh, xp, job.kp_cap, st);
-    ctx->launches++;
-    if (e != cudaSuccess) return cuda_error(ctx, e, "extrema_emit");
-  }
+  int max_rows = 0;
+  for (int i = 0; i < n; ++i) max_rows = std::max(max_rows, job.plans[i].total_rows);
+  e = launch_extrema_emit(job.d_plans, n, max_rows, xp, job.kp_cap, st);
+  ctx->launches++;
+  if (e != cudaSuccess) return cuda_error(ctx, e, "extrema_emit");
   }
   if (stop_after_keypoints) return PSIFT_OK;
   {
