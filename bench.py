@@ -40,12 +40,12 @@ OCTAVES, SCALES, THRESH, MAX_FEATURES = 4, 3, 0.015, 4096
 METRIC = "1080p SIFT detect+describe images/s"
 WORKLOAD = ("1920x1080 u8 blob images (2000 blobs, sigma U(1.5,20), N(0,3) noise); "
             "SiftConfig octaves=4 scales=3 threshold=0.015 upsample=on, cap 4096")
-L2_NOTE = "no flush: per-step working set (~0.5 GB of scale-space planes per image) >> 126 MB L2"
-# DRAM bytes per blur_level_kernel launch, averaged over the 21 launches of one step:
-# one ncu capture at batch 2 (826.2 MB read + written over 21 launches), scaled by 4 to
+L2_NOTE = "no flush: per-step working set (~0.27 GB of scale-space planes per image) >> 126 MB L2"
+# DRAM bytes per blur launch, averaged over the 21 launches of one step: one ncu capture
+# at batch 4 (1100.6 MB read + written over all blur launches of a step), scaled by 2 to
 # the 8 images of a step here (traffic grows with the images processed).  Writes of the
 # small octaves stay in L2 past the kernel's end, so this under-counts writes.
-NCU_TRAFFIC_BLUR_LEVEL = 4 * 826.17e6 / 21
+NCU_TRAFFIC_BLUR_LEVEL = 2 * 1100.64e6 / 21
 
 
 def peaks(key="hbm_gbs"):
@@ -125,8 +125,8 @@ def pyramid_bytes_per_image(h: int, w: int) -> tuple[float, int]:
     """Algorithmic HBM bytes of the pyramid stage for one image, and its launch count.
 
     Octave-0 base: read u8 image (W*H), write G0 (4 B/px).  Each blur level:
-    read G[s-1], write G[s], write D[s-1] (12 B/px); the level that seeds the
-    next octave also writes its base (4 B per next-octave px).
+    read G[s-1], write G[s] (8 B/px; the DoG planes are not stored); the level that
+    seeds the next octave also writes its base (4 B per next-octave px).
     """
     hh, ww = 2 * h, 2 * w
     total = float(h * w) + 4.0 * hh * ww
@@ -135,7 +135,7 @@ def pyramid_bytes_per_image(h: int, w: int) -> tuple[float, int]:
         if hh < 3 or ww < 3:
             break
         p = hh * ww
-        total += (SCALES + 2) * 12.0 * p
+        total += (SCALES + 2) * 8.0 * p
         launches += SCALES + 2
         nh, nw = hh // 2, ww // 2
         if o + 1 < OCTAVES and nh >= 3 and nw >= 3:
@@ -152,12 +152,13 @@ def _blur_radius(sigma: float) -> int:
 
 def pyramid_fp32_ops_per_image(h: int, w: int) -> tuple[float, float]:
     """FP32 lane operations of the pyramid stage for one image: (reference rounding,
-    single rounding).  Each blur tap is a rounded multiply and a rounded add (one
-    fused multiply-add in the single-rounding mode); the horizontal pass of a 64 x 64
-    tile also covers the 2R halo rows, so it costs (64 + 2R) / 64 of the vertical
-    one; the DoG is one subtraction per pixel; the octave base adds the bilinear
-    upsampling's three adds and a multiply.  Radii of the schedule's incremental
-    sigmas (base 1.6, the input's 0.5 doubled by the upsampling)."""
+    single rounding).  The octave base (64 x 64 tiles): a rounded multiply and a rounded
+    add per tap (one fused multiply-add in the single-rounding mode), the horizontal pass
+    over the 2R halo rows too, and the bilinear upsampling's three adds and a multiply.
+    A level (64-column strips): R + 1 products and 2R adds per pixel and pass (symmetric
+    taps share their products; 2R + 1 fused multiply-adds in the single-rounding mode),
+    the horizontal pass over the 2R rows that a segment recomputes too.  Radii of the
+    schedule's incremental sigmas (base 1.6, the input's 0.5 doubled by the upsampling)."""
     k = np.float32(2.0) ** (np.float32(1.0) / np.float32(SCALES))
     radii, prev = [], np.float32(1.6)
     for s in range(1, SCALES + 3):
@@ -179,8 +180,10 @@ def pyramid_fp32_ops_per_image(h: int, w: int) -> tuple[float, float]:
         if hh < 3 or ww < 3:
             break
         for r in radii:
-            ref += hh * ww * (per_px(r, False) + 1.0)
-            fused += hh * ww * (per_px(r, True) + 1.0)
+            rows = 2 * (64 // (2 * r) * (2 * r))  # input rows of a segment
+            passes = 1.0 + rows / (rows - 2 * r)
+            ref += hh * ww * passes * (3 * r + 1)
+            fused += hh * ww * passes * (2 * r + 1)
         hh, ww = hh // 2, ww // 2
     return ref, fused
 
@@ -1223,7 +1226,7 @@ def run_ours(args):
                     "one_thread_images_per_s": e2e_single,
                     "single_image_api_images_per_s": B / single_s,
                     "single_image_api_4_host_threads_images_per_s": B / single4_s},
-            "roofline": {"kernel": "blur_level_kernel (pyramid: blur + DoG + decimation)", "bound": "hbm",
+            "roofline": {"kernel": "blur_strip_kernel / blur_level_kernel (pyramid: blur + decimation)", "bound": "hbm",
                          "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "peak_source": peak_kind, "traffic": NCU_TRAFFIC_BLUR_LEVEL,
                          "algorithmic_bytes_per_launch": bytes_per_launch,
