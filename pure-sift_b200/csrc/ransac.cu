@@ -753,7 +753,9 @@ static __device__ __forceinline__ bool h_inlier(const float4 p, const double* H,
 // is certain for |(U, V)| <= thr |w| - G and excluded for |(U, V)| >= thr |w| + G, and
 // 2 thr |w| G <= k (thr w)^2 + G^2 / k, for any k, turns both into
 //   U^2 + V^2 <= w^2 lo.x + lo.y    and    U^2 + V^2 >= w^2 hi.x + hi.y.
-// In between, for values too large and for NaN the f64 test decides.
+// In between, for values too large and for NaN the f64 test decides: there lo is (-1, -1),
+// below every sum of squares (also of w = U = V = 0, which f32 rounding does give), and hi
+// is NaN.
 static __device__ float4 h_band(const RShared& S, const double* H) {
   const double Qx = __uint_as_float(S.coord_max[0]), Qy = __uint_as_float(S.coord_max[1]), T = __uint_as_float(S.coord_max[2]);
   const double Bx = fabs(H[0]) * Qx + fabs(H[1]) * Qy + fabs(H[2]);
@@ -762,7 +764,7 @@ static __device__ float4 h_band(const RShared& S, const double* H) {
   const double M = Bx + By + T * Bw, thr2 = S.tsq_d;  // Bx + By >= max(Bx, By), and holds a NaN
   const double nan = __longlong_as_double(0x7ff8000000000000ll);
   if (!(M < 1e15) || !(Bw < 1e15) || !(Qx < 1e15) || !(Qy < 1e15) || !(T < 1e15) || !(thr2 < 1e7))
-    return make_float4(-1.0f, 0.0f, (float)nan, 0.0f);
+    return make_float4(-1.0f, -1.0f, (float)nan, 0.0f);
   const double thr = sqrt(thr2);
   const double G = 1.01 * (thr * (3.1 * 0x1p-24 * Bw + 2e-9) + 6.0 * 0x1p-24 * M);
   const double k = fmin(fmax(G / thr, 0x1p-20), 0.5), s = 0x1p-20;  // s: the f32 roundings of the test itself
