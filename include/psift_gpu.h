@@ -97,6 +97,8 @@ const char* psift_last_error(const psift_ctx* ctx);
 uint64_t psift_ctx_launch_count(const psift_ctx* ctx);
 /* The context's CUDA stream (cudaStream_t) for event timing / interop. */
 void* psift_ctx_stream(const psift_ctx* ctx);
+/* Waits for the context's stream.  PSIFT_ERR_TIMEOUT if a wait on the device gave up in a
+ * psift_hamming_topk_dev queued since the last call (its lists lack codes). */
 psift_status psift_ctx_synchronize(psift_ctx* ctx);
 /* Optional per-stage device timing (CUDA events on the context stream).
  * Stages: 0 pyramid (octave base + blur/DoG levels), 1 extrema (mark, scan,
@@ -461,7 +463,9 @@ psift_status psift_hamming_votes(psift_ctx* ctx, const uint64_t* query_codes, ui
 /* Per query, the k (<= 64) catalog codes nearest in Hamming distance, ordered by
  * (distance, catalog index); missing entries are 0xFFFFFFFF.  No counterpart in
  * the reference (its shortlist is per entry); used to shortlist catalogs of
- * millions of descriptors before an exact re-rank. */
+ * millions of descriptors before an exact re-rank.  A wait on the device that gives up
+ * is PSIFT_ERR_TIMEOUT: from psift_hamming_topk, or, after psift_hamming_topk_dev (which
+ * does not wait), from the next psift_ctx_synchronize or psift_hamming_topk. */
 psift_status psift_hamming_topk(psift_ctx* ctx, const uint64_t* query_codes, uint32_t nq,
                                 const uint64_t* catalog_codes, uint64_t ncat, uint32_t k,
                                 uint32_t* idx, uint32_t* dist);

@@ -191,7 +191,8 @@ psift_status psift_hamming_topk_dev(psift_ctx* ctx, const uint64_t* q_codes, uin
   uint8_t* scratch = (uint8_t*)arena_alloc(ctx, topk_scratch((int)nq, block));
   StageScope sc(ctx, STAGE_HAMMING);
   const cudaError_t e = launch_topk(q_codes, (int)nq, cat_codes, (long long)ncat, (int)k, block, scratch, idx, dist,
-                                    ctx->num_sms, ctx->d_error, &ctx->launches, ctx->stream);
+                                    ctx->num_sms, ctx->d_error + 2, &ctx->launches, ctx->stream);
+  ctx->shortlist_queued = true;
   if (e != cudaSuccess) return cuda_error(ctx, e, "hamming_topk");
   return PSIFT_OK;
 }
@@ -212,8 +213,11 @@ psift_status psift_hamming_topk(psift_ctx* ctx, const uint64_t* q_codes, uint32_
   if ((st = h2d(ctx, d_cat, cat_codes, (size_t)ncat * 16)) != PSIFT_OK) return st;
   st = psift_hamming_topk_dev(ctx, d_q, nq, d_cat, ncat, k, d_idx, d_dist);
   if (st != PSIFT_OK) return st;
+  uint32_t word = 0;
+  PSIFT_CUDA_TRY(ctx, cudaMemcpyAsync(&word, ctx->d_error + 2, sizeof word, cudaMemcpyDeviceToHost, ctx->stream));
   PSIFT_CUDA_TRY(ctx, cudaMemcpyAsync(idx, d_idx, (size_t)nq * k * 4, cudaMemcpyDeviceToHost, ctx->stream));
-  return d2h_sync(ctx, dist, d_dist, (size_t)nq * k * 4);
+  if ((st = d2h_sync(ctx, dist, d_dist, (size_t)nq * k * 4)) != PSIFT_OK) return st;
+  return shortlist_status(ctx, word);
 }
 
 psift_status psift_l2_rerank_dev(psift_ctx* ctx, const float* q_desc, uint32_t nq, const float* cat_desc,

@@ -187,6 +187,13 @@ psift_status pinned_reserve(psift_ctx* ctx, size_t bytes) {
   return PSIFT_OK;
 }
 
+psift_status shortlist_status(psift_ctx* ctx, uint32_t word) {
+  ctx->shortlist_queued = false;
+  if (!(word & kErrTimeout)) return PSIFT_OK;
+  PSIFT_CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_error + 2, 0, sizeof(uint32_t), ctx->stream));
+  return set_error(ctx, PSIFT_ERR_TIMEOUT, "hamming_topk: device wait timed out");
+}
+
 // The context's streams and events, as far as they exist.
 static void destroy_streams(psift_ctx* ctx) {
   for (cudaEvent_t e : {ctx->ev_fork, ctx->ev_join, ctx->ev_tail[0], ctx->ev_tail[1]})
@@ -268,8 +275,11 @@ void* psift_ctx_stream(const psift_ctx* ctx) { return ctx ? (void*)ctx->stream :
 
 psift_status psift_ctx_synchronize(psift_ctx* ctx) {
   if (!ctx) return PSIFT_ERR_INVALID_ARGUMENT;
+  uint32_t word = 0;
+  if (ctx->shortlist_queued)
+    PSIFT_CUDA_TRY(ctx, cudaMemcpyAsync(&word, ctx->d_error + 2, sizeof word, cudaMemcpyDeviceToHost, ctx->stream));
   PSIFT_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-  return PSIFT_OK;
+  return psift::shortlist_status(ctx, word);
 }
 
 psift_status psift_ctx_enable_graphs(psift_ctx* ctx, int enable) {

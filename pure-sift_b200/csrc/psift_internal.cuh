@@ -77,8 +77,10 @@ struct psift_ctx {
   psift::DeviceArena stitch;  // panorama: images, features, matches (held across the entries it calls)
   psift::PinnedBuffer pinned;
   int num_sms = 148;
-  // Device status words: [0] error bits (kErr* below), [1] re-rank fallback rows.
+  // Device status words: [0] error bits (kErr* below), [1] re-rank fallback rows, [2] error
+  // bits of the Hamming shortlist (no entry but those that report them clears these).
   uint32_t* d_error = nullptr;
+  bool shortlist_queued = false;  // a shortlist was queued whose bits were not read yet
   psift::StageTimer timer;
   // CUDA graphs of the device batch path, keyed by launch geometry: a key seen
   // once runs eagerly, the second time it is captured, afterwards replayed.
@@ -132,6 +134,9 @@ cudaError_t ensure_smem_attr(const void* func, size_t bytes);
 // Autotuner of the matchers' work decomposition (match_api.cu); appends
 // (path, ms per candidate, chosen) per path to report.
 psift_status autotune_match(psift_ctx* ctx, uint32_t n_desc, uint32_t n_pairs, std::vector<double>& report);
+// After the stream is synchronised: `word` is the shortlist's error word as copied to the
+// host before (ctx.cu); PSIFT_ERR_TIMEOUT once per expired wait, the word cleared.
+psift_status shortlist_status(psift_ctx* ctx, uint32_t word);
 // Statistics of summarize_tracking over the masked matches (ransac_api.cu).
 void tracking_stats(const psift_match* m, uint32_t n, const uint8_t* mask, const float* q_scale,
                     const float* q_ori, const float* t_scale, const float* t_ori, psift_tracking_summary* out);
