@@ -186,7 +186,8 @@ psift_status psift_hamming_topk_dev(psift_ctx* ctx, const uint64_t* q_codes, uin
   if (ncat >= 0xFFFFFFFFull) return set_error(ctx, PSIFT_ERR_INVALID_ARGUMENT, "catalog larger than 2^32-1 codes");
   // 8192 queries at a time (8 KB of candidates each); fewer when the device is that full
   int block = 8192;
-  while ((st = arena_reserve(ctx, topk_scratch((int)nq, block) + 4096)) != PSIFT_OK && block > 128) block /= 8;
+  while ((st = arena_reserve(ctx, topk_scratch((int)nq, block) + 4096)) == PSIFT_ERR_OUT_OF_MEMORY && block > 128)
+    block /= 8;
   if (st != PSIFT_OK) return st;
   uint8_t* scratch = (uint8_t*)arena_alloc(ctx, topk_scratch((int)nq, block));
   StageScope sc(ctx, STAGE_HAMMING);

@@ -1290,7 +1290,7 @@ psift_status run_fundamental(psift_ctx* ctx, const psift_fundamental_job* jobs, 
     size_t bytes = sizeof(FundJob) * (size_t)n + 4096;
     for (int i = 0; i < n; ++i) bytes += (56 + 8 * (size_t)ctas) * (size_t)jobs[i].n + 4 * 256;
     if ((st = arena_reserve(ctx, bytes)) == PSIFT_OK) break;
-    if (ctas == 1) return st;
+    if (st != PSIFT_ERR_OUT_OF_MEMORY || ctas == 1) return st;
     ctas = 1;  // a row of terms per CTA does not fit: one CTA per set
   }
   FundJob* d_jobs = (FundJob*)arena_alloc(ctx, sizeof(FundJob) * n);

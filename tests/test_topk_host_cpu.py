@@ -20,7 +20,7 @@ def harness(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("scenario", ["timeout"])
+@pytest.mark.parametrize("scenario", ["timeout", "memory"])
 def test_failures_reach_the_caller(harness, scenario):
     r = subprocess.run([harness, scenario], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stderr

@@ -109,12 +109,41 @@ static int timeout_reported(psift_ctx* ctx) {
   return 0;
 }
 
+// Queries are taken in smaller blocks when the device is short of memory, and only then.
+static int smaller_blocks(psift_ctx* ctx) {
+  std::vector<uint64_t> q(2 * 8192);
+  std::vector<uint32_t> idx(8192), dist(8192);
+  uint64_t c[2] = {3, 4};
+  g_malloc_limit = 32u << 20;
+  CHECK(psift_hamming_topk_dev(ctx, q.data(), 8192, c, 1, 1, idx.data(), dist.data()) == PSIFT_OK);
+  CHECK(g_launches == 1 && g_block == 1024);
+  g_malloc_limit = 4u << 20;
+  psift_ctx* fresh = nullptr;
+  CHECK(psift_ctx_create(0, &fresh) == PSIFT_OK);
+  CHECK(psift_hamming_topk_dev(fresh, q.data(), 8192, c, 1, 1, idx.data(), dist.data()) == PSIFT_OK);
+  CHECK(g_launches == 2 && g_block == 128);
+  psift_ctx_destroy(fresh);
+  g_malloc_limit = 1u << 20;
+  CHECK(psift_ctx_create(0, &fresh) == PSIFT_OK);
+  CHECK(psift_hamming_topk_dev(fresh, q.data(), 8192, c, 1, 1, idx.data(), dist.data()) == PSIFT_ERR_OUT_OF_MEMORY);
+  // any other failure is returned at once
+  g_malloc_limit = ~(size_t)0;
+  g_sync_result = cudaErrorLaunchFailure;
+  const int before = g_syncs;
+  CHECK(psift_hamming_topk_dev(fresh, q.data(), 8192, c, 1, 1, idx.data(), dist.data()) == PSIFT_ERR_CUDA);
+  CHECK(g_syncs == before + 1 && g_launches == 2);
+  g_sync_result = cudaSuccess;
+  psift_ctx_destroy(fresh);
+  return 0;
+}
+
 int main(int argc, char** argv) {
   psift_ctx* ctx = nullptr;
   CHECK(psift_ctx_create(0, &ctx) == PSIFT_OK);
   CHECK(argc == 2);
   int rc = 2;
   if (!std::strcmp(argv[1], "timeout")) rc = timeout_reported(ctx);
+  if (!std::strcmp(argv[1], "memory")) rc = smaller_blocks(ctx);
   psift_ctx_destroy(ctx);
   return rc;
 }
