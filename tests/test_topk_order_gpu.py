@@ -1,0 +1,117 @@
+"""The Hamming shortlist does not depend on the catalog's order: lists and time of catalogs
+whose near codes lie together, and lists where a part's candidates overflow."""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+import oracle as O
+import psift
+
+pytestmark = pytest.mark.gpu
+
+
+def _codes(rng, n):
+    return rng.integers(0, 2 ** 64, (n, 2), dtype=np.uint64)
+
+
+def _flip(rng, a, bits):
+    a = a.copy()
+    for _ in range(bits):
+        b = rng.integers(0, 128, len(a)).astype(np.uint64)
+        a[np.arange(len(a)), (b >> np.uint64(6)).astype(np.int64)] ^= np.uint64(1) << (b & np.uint64(63))
+    return a
+
+
+def _scenes(rng, ncat, nq, size, bits=16):
+    """A catalog scene after scene (`size` noisy copies of a code each), queries out of some."""
+    centres = _codes(rng, -(-ncat // size))
+    return (_flip(rng, np.repeat(centres, size, 0)[:ncat], bits),
+            _flip(rng, centres[rng.integers(0, len(centres), nq)], bits))
+
+
+def _check(q, c, k, ctx=None):
+    gi, gd = psift.hamming_topk(q, c, k, ctx=ctx)
+    ri, rd = O.hamming_topk(q, c, k)
+    np.testing.assert_array_equal(gd, rd)
+    np.testing.assert_array_equal(gi, ri)
+
+
+# catalogs that end inside a unit of 8 codes, in any part of the order
+@pytest.mark.parametrize("ncat", [2050, 2056, 2057, 2063, 16384, 16390, 16393, 40001, 131079, 150007])
+@pytest.mark.parametrize("size", [300, 9000])
+def test_lists_of_catalogs_in_scene_order(ncat, size):
+    rng = np.random.default_rng(ncat + size)
+    c, q = _scenes(rng, ncat, 70, size)
+    q[0] = c[-1]
+    q[1] = 0  # a short unit's missing codes are not codes
+    for k in (1, 64):
+        _check(q, c, k)
+
+
+def test_nearest_codes_last_and_first():
+    rng = np.random.default_rng(8)
+    c, q = _codes(rng, 50003), _codes(rng, 3)
+    d = np.bitwise_count(c ^ q[0]).sum(1)
+    far_first = np.ascontiguousarray(c[np.argsort(-d.astype(np.int64), kind="stable")])
+    for cat in (far_first, far_first[::-1].copy()):
+        _check(q, cat, 64)
+
+
+def test_time_does_not_depend_on_the_order():
+    # 5 scenes of 80,000 codes: one order by scene, one shuffled
+    import torch
+    rng = np.random.default_rng(9)
+    c, q = _scenes(rng, 400000, 512, 80000)
+    ctx = psift.Context(0)
+    stream = torch.cuda.ExternalStream(ctx.lib.psift_ctx_stream(ctx.handle))
+    dq = torch.from_numpy(q.view(np.int64)).cuda()
+    out = torch.zeros((2, len(q), 64), dtype=torch.int32, device="cuda")
+    ms = []
+    for order in (rng.permutation(len(c)), np.arange(len(c))):
+        dc = torch.from_numpy(np.ascontiguousarray(c[order]).view(np.int64)).cuda()
+        torch.cuda.synchronize()
+        best = 1e9
+        for _ in range(6):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record(stream)
+            ctx.check(ctx.lib.psift_hamming_topk_dev(ctx.handle, C.c_void_p(dq.data_ptr()), len(q),
+                                                     C.c_void_p(dc.data_ptr()), len(c), 64,
+                                                     C.c_void_p(out[0].data_ptr()), C.c_void_p(out[1].data_ptr())))
+            b.record(stream)
+            b.synchronize()
+            best = min(best, a.elapsed_time(b))
+        ms.append(best)
+    ctx.close()
+    assert ms[1] < 2 * ms[0], ms
+
+
+def _last_part(tmp_path, ncat, nq, k):
+    """The codes of the last part of the order (hamming_order.cuh)."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    exe = str(tmp_path / "order")
+    subprocess.run(["g++", "-std=c++17", "-I", os.path.join(root, "pure-sift_b200", "csrc"),
+                    os.path.join(root, "tests", "hamming_order.cpp"), "-o", exe], check=True)
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    out = subprocess.run([exe, "units", str(ncat), str(nq), str(k), str(sms)], capture_output=True, text=True, check=True).stdout
+    codes = (8 * np.array(out.split(), np.int64)[:, None] + np.arange(8)).ravel()
+    return codes[codes < ncat]
+
+
+@pytest.mark.parametrize("equal", [False, True])
+@pytest.mark.parametrize("k", [1, 40, 64])
+def test_candidates_that_overflow_a_part(tmp_path, equal, k):
+    # every code of the last part nearer to the first queries than all before it
+    rng = np.random.default_rng(10)
+    ncat = 30005
+    c, q = _codes(rng, ncat), _codes(rng, 80)
+    idx = _last_part(tmp_path, ncat, len(q), k)
+    assert len(idx) > 8000
+    near = np.repeat(q[:1], len(idx), 0)
+    c[idx] = near if equal else _flip(rng, near, 9)
+    c[idx[5000:5100]] = q[0] ^ np.uint64(1)
+    q[1], q[2], q[3] = q[0], ~q[0], q[0] ^ np.uint64(3)
+    _check(q, c, k)
