@@ -35,7 +35,7 @@ psift_status run_batch(psift_ctx* ctx, const psift_ransac_job* jobs, int n, cons
   size_t bytes = sizeof(RansacJob) * n + 4096;
   for (int i = 0; i < n; ++i) {
     const size_t m = jobs[i].n;
-    bytes += 8 * m + 8 * m + 4 * m + 16 * m + 32 * m + 6 * 256;
+    bytes += 8 * m + 4 * m + 16 * m + 4 * 256;
   }
   psift_status st = arena_reserve(ctx, bytes);
   if (st != PSIFT_OK) return st;
@@ -57,16 +57,14 @@ psift_status run_batch(psift_ctx* ctx, const psift_ransac_job* jobs, int n, cons
     R.homography = homography ? 1 : 0;
     R.weights = J.sampling_weights;
     R.cdf = (double*)arena_alloc(ctx, 8 * m + 8);
-    R.err = (double*)arena_alloc(ctx, 8 * m + 8);
     R.list = (int*)arena_alloc(ctx, 4 * m + 4);
     R.xy = (float4*)arena_alloc(ctx, 16 * m + 16);
-    R.pts = (double*)arena_alloc(ctx, 32 * m + 32);
     R.mask = J.inlier_mask;
     R.model = J.model;
     R.has_model = J.has_model;
     R.count = (int*)J.inlier_count;
     R.iters = (int*)J.iterations;
-    if (!R.pts) return set_error(ctx, PSIFT_ERR_INTERNAL, "ransac workspace carve overflow");
+    if (!R.xy) return set_error(ctx, PSIFT_ERR_INTERNAL, "ransac workspace carve overflow");
   }
   PSIFT_CUDA_TRY(ctx, cudaMemcpyAsync(d_jobs, hj.data(), sizeof(RansacJob) * n, cudaMemcpyHostToDevice, ctx->stream));
   StageScope sc(ctx, STAGE_RANSAC);

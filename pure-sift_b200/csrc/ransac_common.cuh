@@ -23,10 +23,8 @@ struct RansacJob {
   const float* weights;     // optional sampling weights replacing 1/clamp(ratio) (guided sampling)
   // scratch (n entries each)
   double* cdf;
-  double* err;
   int* list;
   float4* xy;               // (query x, query y, target x, target y) per match
-  double* pts;              // 4 per match: the current inlier list's coordinates, gathered
   // outputs
   uint8_t* mask;
   float* model;             // similarity: a, b, tx, ty, scale, rotation_deg; homography: 9 (row-major)
