@@ -984,7 +984,10 @@ static __device__ void run(const FundJob& J0, FShared& S) {
 
     while (S.iter < S.max_iters) {
       // 1. samples of the next iterations (thread 0 walks the resolved draws)
-      const int want = min(kFB * ctas, S.max_iters - S.iter);
+      // The first batch stops at the least number of iterations, which is all that a set of
+      // few outliers takes: 1 / 49 / 140 sets of 100 clean matches 526 / 554 / 630 us, 1226 /
+      // 1044 / 858 when it was as large as the later ones; sets of half outliers pay up to 3 %.
+      const int want = min(kFB * ctas, (S.iter < J.min_iters ? J.min_iters : S.max_iters) - S.iter);
       if (t == 0) S.nb = 0;
       __syncthreads();
       while (true) {

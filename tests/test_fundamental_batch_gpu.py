@@ -1,0 +1,27 @@
+"""The fundamental-matrix estimation of sets with few outliers ends after the least number of
+iterations (64), and no more samples are drawn, fitted and counted for it: the default budget
+costs what a budget of 64 does."""
+import numpy as np
+import pytest
+
+import psift
+import synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("sets", [1, 60, 120])
+def test_budget_beyond_the_least_is_not_paid_for(sets):
+    ctx = psift.Context(0)
+    m = [synth.epipolar_matches(100, 0.0, 50 + k % 3)[0] for k in range(sets)]
+    best, results = [], []
+    for opt in (psift.FundamentalRansacOptions(max_iters=64), psift.FundamentalRansacOptions()):
+        runs = [psift.fundamental_batch(m, opt, ctx, timing=True) for _ in range(8)]
+        best.append(min(ms for _, ms in runs))
+        results.append(runs[0][0])
+    for (mask, f, iters), (mask64, f64, iters64) in zip(*reversed(results)):
+        assert iters == iters64 == 64
+        np.testing.assert_array_equal(mask, mask64)
+        np.testing.assert_array_equal(f, f64)
+    ctx.close()
+    assert best[1] < 1.15 * best[0], best
