@@ -29,8 +29,8 @@ cudaError_t launch_blur(int mode, const float* taps_host, int radius, const Imag
                         uint32_t* err = nullptr);
 cudaError_t launch_extrema_mark(const ImagePlan* plans, int n, int octave, int max_h, int max_w,
                                 const ExtremaParams& prm, cudaStream_t st);
-cudaError_t launch_dog_plane(const float* lower, const float* upper, long long pitch, int h, int w, float* out,
-                             cudaStream_t st);
+cudaError_t launch_dog_planes(const float* g, long long plane_stride, int slices, long long pitch, int h, int w,
+                              float* out, cudaStream_t st);
 cudaError_t launch_row_scan(const ImagePlan* plans, int n, uint32_t kp_cap, uint32_t* err, cudaStream_t st);
 cudaError_t launch_extrema_emit(const ImagePlan* plans, int n, int max_rows, const ExtremaParams& prm, uint32_t kp_cap,
                                 cudaStream_t st);
@@ -421,7 +421,7 @@ psift_status launch_detect(psift_ctx* ctx, DetectJob& job, const psift_sift_conf
   return PSIFT_OK;
 }
 
-// Octave base + blur/DoG levels only (used by the descriptor-only path).
+// Octave base + blur levels only (the descriptor-only path and psift_build_pyramid).
 psift_status launch_pyramid_only(psift_ctx* ctx, DetectJob& job, const psift_sift_config& cfg) {
   cudaStream_t st = ctx->stream;
   const int n = job.n;
@@ -1167,8 +1167,8 @@ psift_status psift_build_pyramid(psift_ctx* ctx, const float* image, uint32_t h,
   void* extra = nullptr;
   psift_sift_config c = *cfg;
   c.max_features = 0;
-  // behind the image: one DoG slice at a time on its way to the caller
-  const size_t dog_bytes = sizeof(float) * (size_t)oct[0].h * oct[0].w;
+  // behind the image: an octave's DoG slices on their way to the caller
+  const size_t dog_bytes = sizeof(float) * (size_t)(S + 2) * oct[0].h * oct[0].w;
   st = build_job(ctx, imgs, c, job, align_up(img_bytes, 256) + dog_bytes, &extra);
   if (st != PSIFT_OK) return st;
   job.plans[0].src = extra;
@@ -1185,13 +1185,11 @@ psift_status psift_build_pyramid(psift_ctx* ctx, const float* image, uint32_t h,
       PSIFT_CUDA_TRY(ctx, cudaMemcpy2DAsync(dst, sizeof(float) * O.w, O.g + (size_t)i * O.plane_stride,
                                             sizeof(float) * O.pitch, sizeof(float) * O.w, O.h,
                                             cudaMemcpyDeviceToHost, ctx->stream));
-    for (int i = 0; i < S + 2; ++i, dst += hw) {
-      const float* lower = O.g + (size_t)i * O.plane_stride;
-      const cudaError_t e = launch_dog_plane(lower, lower + O.plane_stride, O.pitch, O.h, O.w, dog, ctx->stream);
-      ctx->launches++;
-      if (e != cudaSuccess) return cuda_error(ctx, e, "dog_plane");
-      PSIFT_CUDA_TRY(ctx, cudaMemcpyAsync(dst, dog, sizeof(float) * hw, cudaMemcpyDeviceToHost, ctx->stream));
-    }
+    const cudaError_t e = launch_dog_planes(O.g, O.plane_stride, S + 2, O.pitch, O.h, O.w, dog, ctx->stream);
+    ctx->launches++;
+    if (e != cudaSuccess) return cuda_error(ctx, e, "dog_planes");
+    PSIFT_CUDA_TRY(ctx, cudaMemcpyAsync(dst, dog, sizeof(float) * hw * (S + 2), cudaMemcpyDeviceToHost, ctx->stream));
+    dst += hw * (S + 2);
   }
   PSIFT_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
   return PSIFT_OK;

@@ -524,9 +524,13 @@ cudaError_t launch_extrema_mark(const ImagePlan* plans, int n, int octave, int m
   return cudaGetLastError();
 }
 
-// One stored DoG slice, G[i+1] - G[i] (psift_build_pyramid hands the slices to the caller).
-__global__ void dog_plane_kernel(const float* __restrict__ lower, const float* __restrict__ upper, long long pitch,
-                                 int h, int w, float* __restrict__ out) {
+// An octave's DoG slices G[i+1] - G[i], i = blockIdx.y, dense one after the other
+// (psift_build_pyramid hands them to the caller).
+__global__ void dog_planes_kernel(const float* __restrict__ g, long long plane_stride, long long pitch, int h, int w,
+                                  float* __restrict__ out) {
+  const float* lower = g + blockIdx.y * plane_stride;
+  const float* upper = lower + plane_stride;
+  out += (long long)blockIdx.y * h * w;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)h * w;
        i += (long long)gridDim.x * blockDim.x) {
     const int y = (int)(i / w), x = (int)(i - (long long)y * w);
@@ -534,10 +538,11 @@ __global__ void dog_plane_kernel(const float* __restrict__ lower, const float* _
   }
 }
 
-cudaError_t launch_dog_plane(const float* lower, const float* upper, long long pitch, int h, int w, float* out,
-                             cudaStream_t st) {
+cudaError_t launch_dog_planes(const float* g, long long plane_stride, int slices, long long pitch, int h, int w,
+                              float* out, cudaStream_t st) {
   const long long blocks = ((long long)h * w + 255) / 256;
-  dog_plane_kernel<<<(unsigned)(blocks < 148 * 32 ? blocks : 148 * 32), 256, 0, st>>>(lower, upper, pitch, h, w, out);
+  dog_planes_kernel<<<dim3((unsigned)(blocks < 148 * 32 ? blocks : 148 * 32), slices), 256, 0, st>>>(g, plane_stride,
+                                                                                                 pitch, h, w, out);
   return cudaGetLastError();
 }
 
