@@ -1662,10 +1662,13 @@ static cudaError_t launch_ransac_t(const RansacJob* jobs, int n_jobs, cudaStream
 // Sets of 2000 to 7640 matches, outliers 10 to 70 %, milliseconds with 512 / 256 threads
 // per set: 128 sets 3.5 / 5.3, 296 5.5 / 6.0, 444 6.9 / 7.1, 500 7.6 / 7.5, 740 10.5 /
 // 9.5, 1024 13.3 / 11.5 (128 threads, four CTAs per SM: 12.0 to 16.7); one set of 470
-// 0.57 / 0.64.
-cudaError_t launch_ransac(const RansacJob* jobs, int n_jobs, int num_sms, cudaStream_t st) {
+// 0.57 / 0.64.  Sets of a few matches (max_n the most) give 512 threads nothing to do but
+// wait for one another: one similarity of 6 on the host 84 / 73 us, of 100 at 60 % outliers
+// 169 / 173; one homography of 6 567 / 503, of 30 570 / 515, of 12 at 60 % 588 / 647.
+cudaError_t launch_ransac(const RansacJob* jobs, int n_jobs, int max_n, int num_sms, cudaStream_t st) {
   if (n_jobs <= 0) return cudaSuccess;
-  return n_jobs <= 3 * num_sms ? launch_ransac_t<512>(jobs, n_jobs, st) : launch_ransac_t<256>(jobs, n_jobs, st);
+  return n_jobs <= 3 * num_sms && max_n > 32 ? launch_ransac_t<512>(jobs, n_jobs, st)
+                                             : launch_ransac_t<256>(jobs, n_jobs, st);
 }
 
 }  // namespace psift

@@ -4,8 +4,10 @@
 #include "psift_internal.cuh"
 #include "ransac_common.cuh"
 
+static int g_max_n = -1;
 namespace psift {
-cudaError_t launch_ransac(const RansacJob* jobs, int n_jobs, int, cudaStream_t) {
+cudaError_t launch_ransac(const RansacJob* jobs, int n_jobs, int max_n, int, cudaStream_t) {
+  g_max_n = max_n;
   for (int i = 0; i < n_jobs; ++i) {  // every array of a set is there, and in the workspace
     std::memset(jobs[i].cdf, 1, sizeof(double) * (size_t)jobs[i].n);
     std::memset(jobs[i].list, 1, sizeof(int) * (size_t)jobs[i].n);
@@ -31,8 +33,13 @@ int main() {
   g_malloc_limit = 28u * n + (2u << 20);
   for (int homography = 0; homography < 2; ++homography)
     CHECK(psift_ransac_batch_dev(ctx, &job, 1, &opt, homography) == PSIFT_OK);
+  CHECK(g_max_n == (int)n);  // what the CTAs' size goes by
+  psift_ransac_job two[2] = {job, job};
+  two[0].n = 33;
+  two[1].n = 2;
+  CHECK(psift_ransac_batch_dev(ctx, two, 2, &opt, 0) == PSIFT_OK && g_max_n == 33);
+  two[0].n = two[1].n = n;
   g_malloc_limit = 1u << 20;
-  const psift_ransac_job two[2] = {job, job};
   CHECK(psift_ransac_batch_dev(ctx, two, 2, &opt, 1) == PSIFT_ERR_OUT_OF_MEMORY);
   psift_ctx_destroy(ctx);
   std::free(m);
