@@ -150,21 +150,31 @@ def _blur_radius(sigma: float) -> int:
     return max(1, int(np.ceil(np.float32(3.0) * np.float32(cs))))
 
 
-def pyramid_fp32_ops_per_image(h: int, w: int) -> tuple[float, float]:
-    """FP32 lane operations of the pyramid stage for one image: (reference rounding,
-    single rounding).  The octave base (64 x 64 tiles): a rounded multiply and a rounded
-    add per tap (one fused multiply-add in the single-rounding mode), the horizontal pass
-    over the 2R halo rows too, and the bilinear upsampling's three adds and a multiply.
-    A level (64-column strips): R + 1 products and 2R adds per pixel and pass (symmetric
-    taps share their products; 2R + 1 fused multiply-adds in the single-rounding mode),
-    the horizontal pass over the 2R rows that a segment recomputes too.  Radii of the
-    schedule's incremental sigmas (base 1.6, the input's 0.5 doubled by the upsampling)."""
+def level_radii() -> list[int]:
+    """Radii of the schedule's incremental sigmas (base 1.6)."""
     k = np.float32(2.0) ** (np.float32(1.0) / np.float32(SCALES))
     radii, prev = [], np.float32(1.6)
     for s in range(1, SCALES + 3):
         target = np.float32(1.6) * k ** s
         radii.append(_blur_radius(np.sqrt(max(target * target - prev * prev, 1e-4))))
         prev = target
+    return radii
+
+
+STRIP_MIN_PIXELS = 6_000_000  # of a level's launch: strips from here, tiles below (pyramid.cu)
+
+
+def pyramid_fp32_ops_per_image(h: int, w: int, n_images: int) -> tuple[float, float]:
+    """FP32 lane operations of the pyramid stage for one image of n_images per launch:
+    (reference rounding, single rounding).  64 x 64 tiles (the octave base and the levels
+    of small launches): a rounded multiply and a rounded add per tap (one fused
+    multiply-add in the single-rounding mode), the horizontal pass over the 2R halo rows
+    too; the base also has the bilinear upsampling's three adds and a multiply.
+    64-column strips (the other levels): R + 1 products and 2R adds per pixel and pass
+    (symmetric taps share their products; 2R + 1 fused multiply-adds in the
+    single-rounding mode), the horizontal pass over the 2R rows that a segment recomputes
+    too.  The base's radius is that of the first sigma less the input's 0.5, doubled by
+    the upsampling."""
     r0 = _blur_radius(np.sqrt(max(1.6 * 1.6 - 1.0, 1e-4)))
 
     def per_px(r: int, fused: bool) -> float:
@@ -179,7 +189,11 @@ def pyramid_fp32_ops_per_image(h: int, w: int) -> tuple[float, float]:
     for o in range(OCTAVES):
         if hh < 3 or ww < 3:
             break
-        for r in radii:
+        for r in level_radii():
+            if n_images * hh * ww < STRIP_MIN_PIXELS:
+                ref += hh * ww * per_px(r, False)
+                fused += hh * ww * per_px(r, True)
+                continue
             rows = 2 * (64 // (2 * r) * (2 * r))  # input rows of a segment
             passes = 1.0 + rows / (rows - 2 * r)
             ref += hh * ww * passes * (3 * r + 1)
@@ -1069,7 +1083,7 @@ def run_ours(args):
     peak, peak_kind = peaks()
     # the same stage against the FP32 pipe: lane operations over the stage time,
     # peak = SMs x 128 FP32 lanes x the SM clock seen under load
-    ops_ref, ops_fused = pyramid_fp32_ops_per_image(HEIGHT, WIDTH)
+    ops_ref, ops_fused = pyramid_fp32_ops_per_image(HEIGHT, WIDTH, B)  # stage timing: one launch of the batch
     n_sms = torch.cuda.get_device_properties(0).multi_processor_count
 
     # The single-rounding blur mode (PSIFT_BLUR_FUSED: one fused multiply-add per
