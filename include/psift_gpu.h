@@ -101,7 +101,7 @@ void* psift_ctx_stream(const psift_ctx* ctx);
  * psift_hamming_topk_dev queued since the last call (its lists lack codes). */
 psift_status psift_ctx_synchronize(psift_ctx* ctx);
 /* Optional per-stage device timing (CUDA events on the context stream).
- * Stages: 0 pyramid (octave base + blur/DoG levels), 1 extrema (mark, scan,
+ * Stages: 0 pyramid (octave base + blur levels), 1 extrema (mark, scan,
  * emit), 2 top-K cap, 3 orientation, 4 descriptors, 5 matching, 6 Hamming,
  * 7 RANSAC, 8 MLP.  psift_ctx_stage_times synchronises the stream and returns
  * the accumulated milliseconds and the number of timed intervals per stage. */

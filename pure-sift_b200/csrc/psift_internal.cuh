@@ -38,7 +38,7 @@ struct PinnedBuffer {
 namespace psift {
 // Stages timed by the optional per-stage CUDA-event timer.
 enum Stage : int {
-  STAGE_PYRAMID = 0,     // octave base + blur/DoG levels
+  STAGE_PYRAMID = 0,     // octave base + blur levels
   STAGE_EXTREMA = 1,     // mark + scan + emit
   STAGE_SELECT = 2,      // top-K cap
   STAGE_ORIENTATION = 3,
