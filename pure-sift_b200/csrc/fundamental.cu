@@ -650,7 +650,7 @@ struct FShared {
   int nb, refill;
   long long tpos, wb;
   // decision flags of the replay
-  int act;
+  int act, at;
   double ev_err;
   int ev_cnt;
   // LO refit
@@ -1121,32 +1121,32 @@ static __device__ void run(const FundJob& J0, FShared& S) {
       }
       cluster.sync();
       auto model = [&](int k) { return cluster.map_shared_rank(&S, (unsigned)(k / share))->F[k % share]; };
-      // 4. the reference's decisions, in order
+      // 4. the reference's decisions, in order: thread 0 goes on until a tie needs errors
       for (int k = 0; k < nb; ++k) {
         if (t == 0) {
-          S.act = 0;  // 0 nothing, 1 stop, 2 tie needs errors
-          if (S.iter >= S.max_iters) {
-            S.act = 1;
-          } else {
+          S.act = 1;  // 1 the batch or the iterations end, 2 sample S.at ties
+          for (; k < nb && S.iter < S.max_iters; ++k) {
             ++S.iter;
-            if (S.sok[k] && S.fok[k]) {
-              const int c = S.cnt[k];
-              if (c > S.best_count) {
-                S.best_count = c;
-                const double* f = model(k);
-                for (int i = 0; i < 9; ++i) S.best[i] = f[i];
-                S.best_err_known = 0;
-                S.have = 1;
-                S.max_iters = adaptive_epipolar(c, n, J.conf, J.min_iters, J.hard_cap);
-              } else if (c == S.best_count) {
-                S.act = 2;
-              }
+            if (!S.sok[k] || !S.fok[k]) continue;
+            const int c = S.cnt[k];
+            if (c > S.best_count) {
+              S.best_count = c;
+              const double* f = model(k);
+              for (int i = 0; i < 9; ++i) S.best[i] = f[i];
+              S.best_err_known = 0;
+              S.have = 1;
+              S.max_iters = adaptive_epipolar(c, n, J.conf, J.min_iters, J.hard_cap);
+            } else if (c == S.best_count) {
+              S.act = 2;
+              S.at = k;
+              break;
             }
           }
         }
         __syncthreads();
         if (S.act == 1) break;
-        if (S.act == 2) {
+        k = S.at;
+        {
           int c;
           double e;
           if (!S.best_err_known) {
