@@ -303,9 +303,10 @@ __global__ void __launch_bounds__(kHThreads, 1)
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             if (m[h] > thr) {  // few lanes: the columns that beat the threshold
-              uint32_t hit = 0;
+              uint32_t hit = 0;  // bit c: the sign of thr - column c (half of it off the pipe that takes the maxima)
 #pragma unroll
-              for (int c = 0; c < 32; ++c) hit |= (__uint_as_float(r[h][c]) > thr ? 1u : 0u) << c;
+              for (int c = 31; c >= 0; --c)
+                hit = __funnelshift_l(__float_as_uint(__fsub_rn(thr, __uint_as_float(r[h][c]))), hit, 1);
               const long long base = c0 + half * kHN + h * 32;
               if (tail && base + 32 > n) hit &= base >= n ? 0u : (1u << (int)(n - base)) - 1u;  // past the part
               uint32_t pos = hit ? atomicAdd(queued, (uint32_t)__popc(hit)) : 0u;
