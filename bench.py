@@ -1115,7 +1115,7 @@ def run_ours(args):
     blur_fused = {
         "value": world * B * args.steps / (fused_ms / 1e3), "unit": "images/s", "ms_per_step": fused_ms / args.steps,
         "stage_ms_per_step": {k: v[0] / reps for k, v in st_f.items() if v[1]},
-        "roofline": {"kernel": "blur_level_kernel, single-rounding taps", "bound": "hbm", "achieved": fused_achieved,
+        "roofline": {"kernel": "blur_strip_kernel / blur_level_kernel, single-rounding taps", "bound": "hbm", "achieved": fused_achieved,
                      "peak": peak, "unit": "GB/s", "frac": fused_achieved / peak, "peak_source": peak_kind,
                      "avg_launch_ms": fused_launch_s * 1e3},
         "note": "PSIFT_BLUR_FUSED: one fused multiply-add per blur tap; error against an f64 run within 0.01 px / "

@@ -628,8 +628,8 @@ __device__ int cubic_roots(double c3, double c2, double c1, double c0, double* r
 // (sampling CDF, refits, outputs).  48 sets of 2000 to 8000 matches, outliers 10 to
 // 60 %: 24.5 ms with 256 threads and 40-byte match records read, 13.9 with 512, packed
 // matches and counts that stop once they cannot reach the incumbent's, 9.97 with
-// clusters of two.  Sets of 800 matches at 40 %: 4.67 ms with one CTA each (100 sets),
-// 3.35 with two (74), 2.73 with three (44).
+// clusters of two, 9.3 with a replay that stops only for ties.  Sets of 800 matches at
+// 40 %: 4.67 ms with one CTA each (100 sets), 3.35 with two (74), 2.73 with three (44).
 template <int THREADS>
 struct FundCta {
 static constexpr int kFThreads = THREADS;

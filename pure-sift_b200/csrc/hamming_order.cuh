@@ -4,7 +4,7 @@
 // what a part adds is about (its codes / codes before it) * k entries only if the codes
 // before it are a fair sample.  Codes in catalog order are not: neighbours belong to one
 // image or scene, and a scene near to a query comes all at once (2,000,000 codes in scenes
-// of 20,000 x 4096 queries took 38.9 ms that way, 1.7 ms in random order; 2.3 and 1.7 like
+// of 20,000 x 4096 queries took 38.9 ms that way, 1.7 ms in random order; 2.2 and 1.6 like
 // this).  So the parts are samples of the whole catalog, spread evenly and off any period:
 // set 0 is all of the catalog's units (8 codes, one 128-byte line), set i + 1 holds one unit
 // of every few consecutive ones of set i, picked by a hash; the smallest set is taken first,
@@ -38,7 +38,7 @@ struct HammingOrder {
   // For a search of `queries` x `k` on `sms` SMs: the first part and the number of further
   // ones with the least estimated time (see part_us).  Against all choices timed on random
   // codes, 4096 to 4 M x 1 to 16384 queries, its choice costs 0.3 % on average, 8 % at most;
-  // e.g. 2 M x 4096 x 64 1726 us as 4 parts of step 4, 1835 as 3 of 7, 1771 as 5 of 4.
+  // e.g. 2 M x 4096 x 64 1636 us as 4 parts of step 4, 1732 as 3 of 7, 1676 as 5 of 4.
   HammingOrder(uint64_t codes, uint32_t queries, uint32_t k, int sms) : step(2), sets(1), first(kFirst[0]) {
     size[0] = (uint32_t)((codes + kUnit - 1) / kUnit);
     double best = 1e300;
