@@ -70,11 +70,11 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) {
 static __constant__ uint8_t kStrictUpper[36] = {1,  2,  3,  4,  5,  6,  7,  8,  11, 12, 13, 14, 15, 16, 17, 21, 22, 23,
                                                 24, 25, 26, 31, 32, 33, 34, 35, 41, 42, 43, 44, 51, 52, 53, 61, 62, 71};
 
-// A CTA's threads, by the number of match sets of a launch.  512 threads fit and count
-// the most hypotheses at a time, which is what a set with many outliers spends its time
-// on, and take a whole SM; the serial parts (replay, sequential sums, the Jacobi of a
-// refit) leave most of them idle, so once there are several sets per SM two CTAs of
-// 256 threads side by side (128 registers, ~100 KB of shared memory) get more done.
+// A CTA's threads, by the match sets of a launch (see launch_ransac).  512 threads fit and
+// count the most hypotheses at a time, which is what a set with many outliers spends its
+// time on, and take a whole SM; the serial parts (replay, sequential sums, the Jacobi of a
+// refit) leave most of them idle, so once there are several sets per SM two CTAs of 256
+// threads side by side (128 registers, ~100 KB of shared memory) or four of 128 get more done.
 template <int THREADS>
 struct RansacCta {
 static constexpr int kRThreads = THREADS;
@@ -1659,16 +1659,28 @@ static cudaError_t launch_ransac_t(const RansacJob* jobs, int n_jobs, cudaStream
   return cudaGetLastError();
 }
 
-// Sets of 2000 to 7640 matches, outliers 10 to 70 %, milliseconds with 512 / 256 threads
-// per set: 128 sets 3.5 / 5.3, 296 5.5 / 6.0, 444 6.9 / 7.1, 500 7.6 / 7.5, 740 10.5 /
-// 9.5, 1024 13.3 / 11.5 (128 threads, four CTAs per SM: 12.0 to 16.7); one set of 470
-// 0.57 / 0.64.  Sets of a few matches (max_n the most) give 512 threads nothing to do but
-// wait for one another: one similarity of 6 on the host 84 / 73 us, of 100 at 60 % outliers
-// 169 / 173; one homography of 6 567 / 503, of 30 570 / 515, of 12 at 60 % 588 / 647.
-cudaError_t launch_ransac(const RansacJob* jobs, int n_jobs, int max_n, int num_sms, cudaStream_t st) {
+// How many threads a set gets.  Microseconds with 512 / 256 / 128 threads:
+// - up to one set per SM, 512: 148 homographies of 100 to 200 matches, outliers 10 to 70 %,
+//   2834 / 3924 / 6407, of 3800 to 7600 3342 / 5264 / 12124.  But a set of up to 32 matches
+//   gives 512 threads nothing to do but wait for one another: 148 of 12 at 10 % outliers 646 /
+//   571 / 665 (one similarity of 6 on the host 84 us, 73 with 256).
+// - up to two sets per SM, 256, so that all run at once: 296 homographies of 100 matches, 10 %,
+//   1079 / 534 / 613; 296 of 1000 to 2000, 10 to 70 %, 3340 / 2961 / 4366.  Where sets differ
+//   much, the longest ones set the time and 512 would still be better (of 100 to 200, 10 to
+//   70 %, 3354 / 4133 / 6560), but half the speed for sets that are alike is worse.
+// - beyond, similarities, which have little for many threads to share, 128, four sets per SM:
+//   444 of 100 matches, 10 %, 238 / 156 / 92, of 1000 to 2000, 10 to 70 %, 1223 / 1017 / 977;
+//   256 for larger sets (592 of 2000 to 4000 2235 / 1744 / 1959).
+// - beyond, homographies 256: 444 of 100 matches, 10 %, 1609 / 1032 / 656, but of 100 to 200, 10
+//   to 70 %, 3996 / 4482 / 6606; 1200 of those 7782 / 6715 / 8076, of 400 to 800 7844 / 6013 /
+//   6527.  Of up to 32 matches 128 from three sets per SM: 1000 of 12, 10 %, 4058 / 2101 / 1449.
+cudaError_t launch_ransac(const RansacJob* jobs, int n_jobs, int n_sim, int max_n, double mean_n, int num_sms,
+                          cudaStream_t st) {
   if (n_jobs <= 0) return cudaSuccess;
-  return n_jobs <= 3 * num_sms && max_n > 32 ? launch_ransac_t<512>(jobs, n_jobs, st)
-                                             : launch_ransac_t<256>(jobs, n_jobs, st);
+  const bool few = max_n <= 32;
+  if (n_jobs <= num_sms && !few) return launch_ransac_t<512>(jobs, n_jobs, st);
+  const bool small = n_sim == n_jobs ? n_jobs > 2 * num_sms && mean_n <= 2000.0 : n_jobs > 3 * num_sms && few;
+  return small ? launch_ransac_t<128>(jobs, n_jobs, st) : launch_ransac_t<256>(jobs, n_jobs, st);
 }
 
 }  // namespace psift

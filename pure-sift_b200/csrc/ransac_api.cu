@@ -13,7 +13,8 @@
 
 namespace psift {
 
-cudaError_t launch_ransac(const RansacJob* jobs, int n_jobs, int max_n, int num_sms, cudaStream_t st);
+cudaError_t launch_ransac(const RansacJob* jobs, int n_jobs, int n_sim, int max_n, double mean_n, int num_sms,
+                          cudaStream_t st);
 
 namespace {
 constexpr uint64_t kSimSeed = 0xD1B54A32D192ED03ull;   // DEFAULT_SIMILARITY_RANSAC_SEED, src/pipeline.rs:172
@@ -34,10 +35,12 @@ psift_status run_batch(psift_ctx* ctx, const psift_ransac_job* jobs, int n, cons
                        int n_sim) {
   size_t bytes = sizeof(RansacJob) * n + 4096;
   int max_n = 0;
+  double total = 0.0;
   for (int i = 0; i < n; ++i) {
     const size_t m = jobs[i].n;
     bytes += 8 * m + 4 * m + 16 * m + 4 * 256;
     max_n = std::max(max_n, (int)m);
+    total += (double)m;
   }
   psift_status st = arena_reserve(ctx, bytes);
   if (st != PSIFT_OK) return st;
@@ -70,7 +73,7 @@ psift_status run_batch(psift_ctx* ctx, const psift_ransac_job* jobs, int n, cons
   }
   PSIFT_CUDA_TRY(ctx, cudaMemcpyAsync(d_jobs, hj.data(), sizeof(RansacJob) * n, cudaMemcpyHostToDevice, ctx->stream));
   StageScope sc(ctx, STAGE_RANSAC);
-  cudaError_t e = launch_ransac(d_jobs, n, max_n, ctx->num_sms, ctx->stream);
+  cudaError_t e = launch_ransac(d_jobs, n, n_sim, max_n, total / n, ctx->num_sms, ctx->stream);
   ctx->launches++;
   if (e != cudaSuccess) return cuda_error(ctx, e, "ransac");
   return PSIFT_OK;

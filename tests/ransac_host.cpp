@@ -4,10 +4,13 @@
 #include "psift_internal.cuh"
 #include "ransac_common.cuh"
 
-static int g_max_n = -1;
+static int g_max_n = -1, g_n_sim = -1;
+static double g_mean_n = -1;
 namespace psift {
-cudaError_t launch_ransac(const RansacJob* jobs, int n_jobs, int max_n, int, cudaStream_t) {
+cudaError_t launch_ransac(const RansacJob* jobs, int n_jobs, int n_sim, int max_n, double mean_n, int, cudaStream_t) {
   g_max_n = max_n;
+  g_n_sim = n_sim;
+  g_mean_n = mean_n;
   for (int i = 0; i < n_jobs; ++i) {  // every array of a set is there, and in the workspace
     std::memset(jobs[i].cdf, 1, sizeof(double) * (size_t)jobs[i].n);
     std::memset(jobs[i].list, 1, sizeof(int) * (size_t)jobs[i].n);
@@ -38,6 +41,8 @@ int main() {
   two[0].n = 33;
   two[1].n = 2;
   CHECK(psift_ransac_batch_dev(ctx, two, 2, &opt, 0) == PSIFT_OK && g_max_n == 33);
+  CHECK(g_n_sim == 2 && g_mean_n == 17.5);
+  CHECK(psift_ransac_batch_dev(ctx, two, 2, &opt, 1) == PSIFT_OK && g_n_sim == 0);
   two[0].n = two[1].n = n;
   g_malloc_limit = 1u << 20;
   CHECK(psift_ransac_batch_dev(ctx, two, 2, &opt, 1) == PSIFT_ERR_OUT_OF_MEMORY);
