@@ -202,16 +202,18 @@ __global__ void __launch_bounds__(256) votes_kernel(const uint4* __restrict__ q,
 
 // Exact FP32 L2^2 re-rank of each query's k candidates (reference summation
 // order), sorted by (d2, index).  One warp per query; its candidates' rows come into
-// shared memory kRerankRows at a time (a row is one coalesced 512-byte asynchronous
-// copy), where lane c sums candidate c.  Bound by the random 512-byte rows: 4096 x 64 of
-// a 2M-row catalog (134 MB) took 147 us with a lane walking each row in global memory.
+// shared memory `turn` at a time, k in equal turns of at most kRerankRows (a row is one
+// coalesced 512-byte asynchronous copy), where lane c sums candidate c; no more shared
+// memory than the turns need, so that few candidates leave room for more warps.  Bound by
+// the random 512-byte rows: 4096 x 64 of a 2M-row catalog (134 MB) 50 us, 147 with a lane
+// walking each row in global memory; 16384 x 1 / 17 / 64 of 500,000 rows 37 / 65 / 124 us
+// (47 / 80 / 128 with 16 rows' memory and turns for every k; 39 / 77 / 256 by walking).
 constexpr int kRerankRows = 16;
 constexpr int kRerankStride = 132;  // floats per staged row: lanes of different rows hit distinct banks
 constexpr int kRerankWarps = 8;
-constexpr size_t kRerankSmem = sizeof(float) * kRerankWarps * kRerankRows * kRerankStride;
 __global__ void __launch_bounds__(32 * kRerankWarps) l2_rerank_kernel(const float* __restrict__ qd, int nq,
                                                                       const float* __restrict__ cd,
-                                                                      const uint32_t* __restrict__ cand, int k,
+                                                                      const uint32_t* __restrict__ cand, int k, int turn,
                                                                       uint32_t* __restrict__ out_idx,
                                                                       float* __restrict__ out_d2) {
   __shared__ unsigned long long s_keys[kRerankWarps][kTopKMax];
@@ -220,11 +222,11 @@ __global__ void __launch_bounds__(32 * kRerankWarps) l2_rerank_kernel(const floa
   const int qi = blockIdx.x * kRerankWarps + warp;
   if (qi >= nq) return;
   unsigned long long* keys = s_keys[warp];
-  float* rows = reinterpret_cast<float*>(s_rows) + warp * kRerankRows * kRerankStride;
+  float* rows = reinterpret_cast<float*>(s_rows) + warp * turn * kRerankStride;
   const float* a = qd + (size_t)qi * 128;
   for (int t = lane; t < kTopKMax; t += 32) keys[t] = ~0ull;
-  for (int t0 = 0; t0 < k; t0 += kRerankRows) {
-    const int nr = min(kRerankRows, k - t0);
+  for (int t0 = 0; t0 < k; t0 += turn) {
+    const int nr = min(turn, k - t0);
     const uint32_t mine = lane < nr ? cand[(long long)qi * k + t0 + lane] : 0xFFFFFFFFu;
     __syncwarp();  // the previous rows are read
     for (int r = 0; r < nr; ++r) {
@@ -333,10 +335,12 @@ cudaError_t launch_popc_probe(int blocks, int iters, uint32_t* out, cudaStream_t
 cudaError_t launch_l2_rerank(const float* qd, int nq, const float* cd, const uint32_t* cand, int k,
                              uint32_t* out_idx, float* out_d2, cudaStream_t st) {
   if (nq <= 0) return cudaSuccess;
-  cudaError_t e = ensure_smem_attr((const void*)l2_rerank_kernel, kRerankSmem);
+  const int turns = (k + kRerankRows - 1) / kRerankRows, turn = (k + turns - 1) / turns;
+  const size_t smem = sizeof(float) * kRerankWarps * turn * kRerankStride;
+  cudaError_t e = ensure_smem_attr((const void*)l2_rerank_kernel, smem);
   if (e != cudaSuccess) return e;
-  l2_rerank_kernel<<<(nq + kRerankWarps - 1) / kRerankWarps, 32 * kRerankWarps, kRerankSmem, st>>>(qd, nq, cd, cand, k,
-                                                                                                 out_idx, out_d2);
+  l2_rerank_kernel<<<(nq + kRerankWarps - 1) / kRerankWarps, 32 * kRerankWarps, smem, st>>>(qd, nq, cd, cand, k, turn,
+                                                                                          out_idx, out_d2);
   return cudaGetLastError();
 }
 

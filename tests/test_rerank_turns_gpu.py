@@ -1,0 +1,51 @@
+"""The exact re-rank's staged turns: results at every number of turns and rows, and no time for
+rows that a call does not have."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import oracle as O
+import psift
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nq", [1, 7, 8, 9, 65])
+@pytest.mark.parametrize("k", [1, 2, 15, 16, 17, 31, 32, 33, 47, 49, 63, 64])
+def test_results(nq, k):
+    rng = np.random.default_rng(nq * 100 + k)
+    q, c = rng.random((nq, 128), dtype=np.float32), rng.random((500, 128), dtype=np.float32)
+    c[100:110] = c[0]  # equal distances: the index decides
+    cand = rng.integers(0, 500, (nq, k)).astype(np.uint32)
+    cand[rng.random((nq, k)) < 0.1] = 0xFFFFFFFF  # no candidate
+    gi, gd = psift.l2_rerank(q, c, cand)
+    ri, rd = O.l2_rerank(q, c, cand)
+    np.testing.assert_array_equal(gi, ri)
+    np.testing.assert_array_equal(gd, rd)
+
+
+def test_time_of_few_candidates():
+    # 16384 queries: memory for 16 rows a warp leaves three CTAs per SM, whatever k is, and a
+    # 17th candidate took a turn of its own
+    import torch
+    ctx = psift.Context(0)
+    stream = torch.cuda.ExternalStream(ctx.lib.psift_ctx_stream(ctx.handle))
+    q, cat = (torch.randn(n, 128, device="cuda") for n in (16384, 500000))
+    us = {}
+    for k in (1, 16, 17):
+        cand = torch.randint(0, 500000, (16384, k), device="cuda", dtype=torch.int32)
+        oi, od = torch.zeros_like(cand), torch.zeros(16384, k, device="cuda")
+        torch.cuda.synchronize()
+        best = 1e9
+        for _ in range(30):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record(stream)
+            p = [C.c_void_p(x.data_ptr()) for x in (q, cat, cand, oi, od)]
+            ctx.check(ctx.lib.psift_l2_rerank_dev(ctx.handle, p[0], 16384, p[1], p[2], k, p[3], p[4]))
+            b.record(stream)
+            b.synchronize()
+            best = min(best, a.elapsed_time(b))
+        us[k] = best * 1e3
+    ctx.close()
+    assert us[1] < 0.64 * us[16] and us[17] < 1.12 * us[16], us
