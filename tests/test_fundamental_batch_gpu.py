@@ -24,4 +24,4 @@ def test_budget_beyond_the_least_is_not_paid_for(sets):
         np.testing.assert_array_equal(mask, mask64)
         np.testing.assert_array_equal(f, f64)
     ctx.close()
-    assert best[1] < 1.15 * best[0], best
+    assert best[1] < 1.25 * best[0], best  # 1.4 to 2.3 when every batch was full

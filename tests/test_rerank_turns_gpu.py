@@ -48,4 +48,4 @@ def test_time_of_few_candidates():
             best = min(best, a.elapsed_time(b))
         us[k] = best * 1e3
     ctx.close()
-    assert us[1] < 0.64 * us[16] and us[17] < 1.12 * us[16], us
+    assert us[1] < 0.67 * us[16] and us[17] < 1.15 * us[16], us  # 0.57 and 1.02; 0.71 and 1.20 before

