@@ -25,3 +25,18 @@ def test_budget_beyond_the_least_is_not_paid_for(sets):
         np.testing.assert_array_equal(f, f64)
     ctx.close()
     assert best[1] < 1.25 * best[0], best  # 1.4 to 2.3 when every batch was full
+
+
+# error terms of a set's ties lie in shared memory up to 10368 matches with 256 threads, 20736 with 512
+@pytest.mark.parametrize("sizes", [(10368, 10369), (20736, 20737), (33, 30000)])
+def test_ties_at_the_end_of_the_staged_terms(sizes):
+    ctx = psift.Context(0)
+    sets = [synth.epipolar_matches(n, 0.0, 70 + n % 5)[0] for n in sizes]
+    opt = psift.FundamentalRansacOptions(max_iters=64)
+    alone = [psift.fundamental_batch([m], opt, ctx)[0] for m in sets]
+    for i, (mask, f, iters) in enumerate(psift.fundamental_batch(sets * 75, opt, ctx)):  # more sets than SMs
+        m1, f1, it1 = alone[i % len(sets)]
+        np.testing.assert_array_equal(mask, m1)
+        np.testing.assert_array_equal(f, f1)
+        assert iters == it1
+    ctx.close()
